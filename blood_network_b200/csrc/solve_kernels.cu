@@ -379,13 +379,17 @@ k_spmv_long(const int* __restrict__ ia, const int* __restrict__ ja, const T* __r
   }
 }
 
+// counter[0]: rows longer than kLongRow, counter[1]: the longest row's length
 __global__ void k_long_rows(const int* __restrict__ ia, int n, int* __restrict__ lrows,
                             int* counter) {
   // warp-aggregated appends (the list is sorted afterwards)
   const int lane = threadIdx.x & 31;
+  int longest = 0;
   for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     const int i = base + threadIdx.x;
-    const bool lng = i < n && ia[i + 1] - ia[i] > kLongRow;
+    const int len = i < n ? ia[i + 1] - ia[i] : 0;
+    longest = max(longest, len);
+    const bool lng = len > kLongRow;
     const unsigned m = __ballot_sync(0xffffffffu, lng);
     if (!m) continue;
     int pos0 = 0;
@@ -393,6 +397,8 @@ __global__ void k_long_rows(const int* __restrict__ ia, int n, int* __restrict__
     pos0 = __shfl_sync(0xffffffffu, pos0, 0);
     if (lng) lrows[pos0 + __popc(m & ((1u << lane) - 1u))] = i;
   }
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  if (lane == 0) atomicMax(counter + 1, longest);
 }
 
 void analyze_rows(const CSR& A, RowLayout& out, cudaStream_t s) {
@@ -404,12 +410,16 @@ void analyze_rows(const CSR& A, RowLayout& out, cudaStream_t s) {
   static const int forced = getenv("BN_SPMV_GROUP") ? atoi(getenv("BN_SPMV_GROUP")) : -1;
   if ((forced >= 0 && forced <= 5) || forced == 8 || forced == 16 || forced == 32)
     out.group = forced;
-  DBuf<int> cnt(1, s);
+  DBuf<int> cnt(2, s);
   cnt.zero();
   out.lrows.alloc(A.n > 0 ? A.n : 1, s);
   if (A.n > 0)
     BN_LAUNCH(k_long_rows, grid_for(A.n, 256), 256, 0, s, A.ia.p, A.n, out.lrows.p, cnt.p);
-  out.nlong = read_scalar(cnt.p, s);
+  int hc[2];
+  cnt.download(hc, 2);
+  BN_CUDA(cudaStreamSynchronize(s));
+  out.nlong = hc[0];
+  out.maxrow = hc[1];
   if (out.nlong > 1) {  // deterministic order
     DBuf<int> tmp_out(out.nlong, s);
     size_t tmp = 0;

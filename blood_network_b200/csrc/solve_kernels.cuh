@@ -50,6 +50,7 @@ struct RowLayout {
   DBuf<int> tiles;  // visiting order of the kRows-row tiles (empty: natural)
   DBuf<int> lrows;
   int nlong = 0;
+  int maxrow = 0;   // entries of the longest row
 };
 void analyze_rows(const CSR& A, RowLayout& out, cudaStream_t s);
 // Visit the row tiles of a matrix in the order of key[first row of tile]

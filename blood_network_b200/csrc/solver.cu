@@ -45,6 +45,18 @@ constexpr double kCapAvgRow = 8.0;  // levels with more entries per row than thi
 constexpr int kCappedRounds = 8;    // colouring rounds on capped levels
 constexpr int kColorLong = 256;     // rows longer than this are coloured by a warp
 constexpr int kColorHuge = 4096;    // ... and longer than this by a block
+// Operators whose longest row passes this many entries run on the packed
+// kernels.  The row-group kernels have one thread (row tiles) or a few lanes
+// walk such a row, and on a coarse operator the launch waits for it: a
+// restriction of 15k rows with rows of some hundred entries took 96 us, packed
+// 8 us.  2M network FP64, whole solve: 29.7 ms without the rule, 27.1 ms with
+// a line at 256 or 128, 27.8 ms at 64 (operators that fit the row groups pay
+// the packing's two barriers); 64 packed networks 30.6, 26.2 at 256-64.
+constexpr int kIrregularRow = 128;
+// On operators beyond this size the long rows hide behind the others, and
+// packing (on the host) costs setup time: 80M entries as the line gained 0.7 %
+// on the 20M network's solve.
+constexpr long long kIrregularNnz = 8000000;
 constexpr int kSmallLevel = 2048;  // levels up to this size (without hub rows) sweep in one block
 // levels with at most this many entries take no split first sweep
 constexpr long long kSmallLevelNnz = 65536;
@@ -691,9 +703,12 @@ void Solver::build_solve_layout() {
       }
       if (use_packed) {  // packings only for the operators that run on them
         Phase ph2("packing", s, l);
-        L.use_pkA = L.layA.nlong > 0;
-        L.use_pkP = L.layP.nlong > 0;
-        L.use_pkR = L.layR.nlong > 0;
+        auto irregular = [](const RowLayout& lay, const CSR& M) {
+          return lay.nlong > 0 || (lay.maxrow > kIrregularRow && M.nnz <= kIrregularNnz);
+        };
+        L.use_pkA = irregular(L.layA, L.Ap);
+        L.use_pkP = irregular(L.layP, L.Pp);
+        L.use_pkR = irregular(L.layR, L.Rp);
         if (L.use_pkA) {
           std::vector<int> ha = host_ia(L.Ap, s);
           L.pkA.build(ha, {make_int2(0, L.Ap.n)}, s);

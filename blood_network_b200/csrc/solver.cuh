@@ -45,7 +45,8 @@ struct Level {
   // the colour classes of Ap (one range per class)
   Packing pkA, pkP, pkR, pkG;
   // which operators run on the packed kernels: those with rows longer than
-  // kLongRow (hub rows); the row-group kernels are faster on the others
+  // kLongRow (hub rows) and the smaller ones with irregular rows
+  // (kIrregularRow, solver.cu); the row-group kernels are faster on the others
   bool use_pkA = false, use_pkP = false, use_pkR = false;
   // Ap split by colour class for the first smoothing sweep from a zero
   // guess (coloured levels on the row-group kernels): AL row i holds the
