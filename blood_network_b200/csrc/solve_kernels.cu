@@ -872,27 +872,58 @@ void vxpby(double* p, const double* z, double b, int n, cudaStream_t s) {
 
 // ---- segmented PCG (independent systems packed block-diagonally)
 // out[k] = sum over the rows of segment k (natural rows ptr[k]..ptr[k+1]-1,
-// held at solve index idx[row]) of u*v: one block per segment, fixed order
+// held at solve index idx[row]) of u*v.  Bound by the latency of the gather
+// idx -> u, v: one block per segment walked its rows alone (64 networks of
+// 5k-60k rows: 140 us a launch on 64 of the 148 SMs).  Each segment is cut
+// into gridDim.y slices of consecutive rows, a block each, four gathers in
+// flight per thread; the slice that arrives last adds the slices' sums in
+// slice order, so the result does not depend on which one that is.
 __global__ void __launch_bounds__(256)
 k_seg_dot(const double* __restrict__ u, const double* __restrict__ v,
           const int* __restrict__ ptr, const int* __restrict__ idx, int nseg,
-          double* __restrict__ out) {
+          double* __restrict__ out, double* part, int* arrived) {
   BN_PDL_ENTRY();
   __shared__ double red[32];
+  const int S = gridDim.y, y = blockIdx.y;
   for (int k = blockIdx.x; k < nseg; k += gridDim.x) {
+    const int lo = ptr[k], len = ptr[k + 1] - lo;
+    const int r0 = lo + (int)((long long)len * y / S), r1 = lo + (int)((long long)len * (y + 1) / S);
     double a = 0.0;
-    for (int r = ptr[k] + threadIdx.x; r < ptr[k + 1]; r += blockDim.x) {
+#pragma unroll 4
+    for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
       const int t = idx[r];
       a += u[t] * v[t];
     }
     const double tot = block_sum(a, red);
-    if (threadIdx.x == 0) out[k] = tot;
+    if (threadIdx.x == 0) {
+      if (S == 1) {
+        out[k] = tot;
+      } else {
+        part[(size_t)k * S + y] = tot;
+        __threadfence();
+        if (atomicAdd(&arrived[k], 1) == S - 1) {
+          __threadfence();
+          double t = 0.0;
+          for (int q = 0; q < S; q++) t += __ldcg(part + (size_t)k * S + q);
+          out[k] = t;
+          arrived[k] = 0;  // for the next launch
+        }
+      }
+    }
     __syncthreads();
   }
 }
+// slices per segment: about four blocks per SM over all segments, at most 64
+// (64 segments: 9 slices; a single one: 64)
+int seg_dot_slices(int nseg) {
+  const int s = nseg > 0 ? 4 * kSMs / nseg : 1;
+  return s < 1 ? 1 : (s > 64 ? 64 : s);
+}
 void seg_dot(const double* u, const double* v, const int* ptr, const int* idx, int nseg,
-             double* out, cudaStream_t s) {
-  if (nseg > 0) BN_LAUNCH_PDL(k_seg_dot, nseg < 4096 ? nseg : 4096, 256, 0, s, u, v, ptr, idx, nseg, out);
+             double* out, const SegDotWork& w, cudaStream_t s) {
+  if (nseg <= 0) return;
+  const dim3 grid(nseg < 4096 ? nseg : 4096, seg_dot_slices(nseg));
+  BN_LAUNCH_PDL(k_seg_dot, grid, 256, 0, s, u, v, ptr, idx, nseg, out, w.part, w.arrived);
 }
 
 // segment of every solve-numbered row: perm[t] is its natural row

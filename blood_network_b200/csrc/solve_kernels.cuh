@@ -105,8 +105,13 @@ void reduce_partials(const double* part, int m, double* out, cudaStream_t s);
 void vaxpy(double* y, const double* u, double a, int n, cudaStream_t s);   // y += a u
 // segmented PCG helpers: segments are natural row ranges ptr[k]..ptr[k+1]-1,
 // idx maps a natural row to its solve index, seg a solve index to its segment
+struct SegDotWork {
+  double* part;  // nseg * seg_dot_slices(nseg)
+  int* arrived;  // nseg, zero between launches
+};
+int seg_dot_slices(int nseg);
 void seg_dot(const double* u, const double* v, const int* ptr, const int* idx, int nseg,
-             double* out, cudaStream_t s);
+             double* out, const SegDotWork& w, cudaStream_t s);
 void seg_of_rows(const int* perm, int n, const int* ptr, int nseg, int* seg, cudaStream_t s);
 void seg_update_xr(double* x, double* r, const double* p, const double* ap, const int* seg,
                    const double* alpha, int n, cudaStream_t s);

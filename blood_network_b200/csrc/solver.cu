@@ -1469,10 +1469,12 @@ int Solver::pcg_segmented(int nseg, const int* d_ptr, const double* d_b, double*
   DevMat<double> A = mat<double>(Asolve_p(), nullptr, &lay_solve());
   const int* perm0 = lv[0]->perm.p;
   const int* inv0 = lv[0]->inv.p;
-  DBuf<int> seg(n0, s), ints((size_t)2 * nseg + 2, s);
+  DBuf<int> seg(n0, s), ints((size_t)3 * nseg + 2, s);
+  DBuf<double> dot_part((size_t)nseg * seg_dot_slices(nseg), s);
   int* active = ints.p;
   int* iters = ints.p + nseg;
   int* flag = ints.p + 2 * nseg;  // [0] block-diagonal check, [1] segments iterating
+  const SegDotWork dw = {dot_part.p, ints.p + 2 * nseg + 2};
   ints.zero();
   seg_of_rows(perm0, n0, d_ptr, nseg, seg.p, s);
   const CSR& Ap = Asolve_p();
@@ -1486,10 +1488,10 @@ int Solver::pcg_segmented(int nseg, const int* d_ptr, const double* d_b, double*
   vpermute<double>(d_b, perm0, n0, b.p, false, s);
   vpermute<double>(d_x, perm0, n0, x.p, false, s);
   spmv<double>(SPMV_RES, A, x.p, b.p, r.p, s);  // r = b - A x
-  seg_dot(b.p, b.p, d_ptr, inv0, nseg, S_(BB), s);
+  seg_dot(b.p, b.p, d_ptr, inv0, nseg, S_(BB), dw, s);
   precond(r.p, z.p);
   BN_CUDA(cudaMemcpyAsync(p.p, z.p, sizeof(double) * n0, cudaMemcpyDeviceToDevice, s));
-  seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZ), s);
+  seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZ), dw, s);
   BN_CUDA(cudaMemcpyAsync(S_(RZ0), S_(RZ), sizeof(double) * nseg, cudaMemcpyDeviceToDevice, s));
   BN_LAUNCH(k_seg_start, grid_for(nseg, 256), 256, 0, s, S_(RZ), nseg, active, iters, flag + 1);
   int nact = read_scalar(flag + 1, s);
@@ -1505,13 +1507,13 @@ int Solver::pcg_segmented(int nseg, const int* d_ptr, const double* d_b, double*
     seg_loop = build_loop_graph(s, [&](cudaGraphConditionalHandle h) {
       capture_direct = true;
       spmv<double>(SPMV_Y, A, p.p, nullptr, ap.p, s);
-      seg_dot(p.p, ap.p, d_ptr, inv0, nseg, S_(PAP), s);
+      seg_dot(p.p, ap.p, d_ptr, inv0, nseg, S_(PAP), dw, s);
       seg_alpha(S_(RZ), S_(PAP), active, nseg, S_(ALPHA), s);
       seg_update_xr(x.p, r.p, p.p, ap.p, seg.p, S_(ALPHA), n0, s);
-      if (relres) seg_dot(r.p, r.p, d_ptr, inv0, nseg, S_(RR), s);
-      if (flexible) seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZON), s);
+      if (relres) seg_dot(r.p, r.p, d_ptr, inv0, nseg, S_(RR), dw, s);
+      if (flexible) seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZON), dw, s);
       precond(r.p, z.p);
-      seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZNEW), s);
+      seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZNEW), dw, s);
       BN_CUDA(cudaMemsetAsync(flag + 1, 0, sizeof(int), s));
       seg_next(S_(RZ), S_(RZNEW), S_(RZON), S_(RR), S_(BB), S_(RZ0), active, iters, S_(BETA),
                nseg, flexible ? 1 : 0, relres, tol, 0, flag + 1, s, ctl.p);
@@ -1539,13 +1541,13 @@ int Solver::pcg_segmented(int nseg, const int* d_ptr, const double* d_b, double*
   } else
   for (iter = 1; iter <= maxiter && nact > 0; iter++) {
     spmv<double>(SPMV_Y, A, p.p, nullptr, ap.p, s);
-    seg_dot(p.p, ap.p, d_ptr, inv0, nseg, S_(PAP), s);
+    seg_dot(p.p, ap.p, d_ptr, inv0, nseg, S_(PAP), dw, s);
     seg_alpha(S_(RZ), S_(PAP), active, nseg, S_(ALPHA), s);
     seg_update_xr(x.p, r.p, p.p, ap.p, seg.p, S_(ALPHA), n0, s);
-    if (relres) seg_dot(r.p, r.p, d_ptr, inv0, nseg, S_(RR), s);
-    if (flexible) seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZON), s);
+    if (relres) seg_dot(r.p, r.p, d_ptr, inv0, nseg, S_(RR), dw, s);
+    if (flexible) seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZON), dw, s);
     precond(r.p, z.p);
-    seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZNEW), s);
+    seg_dot(r.p, z.p, d_ptr, inv0, nseg, S_(RZNEW), dw, s);
     BN_CUDA(cudaMemsetAsync(flag + 1, 0, sizeof(int), s));
     seg_next(S_(RZ), S_(RZNEW), S_(RZON), S_(RR), S_(BB), S_(RZ0), active, iters, S_(BETA),
              nseg, flexible ? 1 : 0, relres, tol, iter, flag + 1, s);
@@ -1555,7 +1557,7 @@ int Solver::pcg_segmented(int nseg, const int* d_ptr, const double* d_b, double*
   }
   // true residual per segment
   spmv<double>(SPMV_RES, A, x.p, b.p, ap.p, s);
-  seg_dot(ap.p, ap.p, d_ptr, inv0, nseg, S_(RR), s);
+  seg_dot(ap.p, ap.p, d_ptr, inv0, nseg, S_(RR), dw, s);
   BN_LAUNCH(k_seg_relres, grid_for(nseg, 256), 256, 0, s, S_(RR), S_(BB), nseg, S_(ALPHA));
   vpermute<double>(x.p, perm0, n0, d_x, true, s);
   cudaEventRecord(ev1, s);

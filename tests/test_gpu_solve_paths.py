@@ -30,3 +30,30 @@ def test_irregular_rows_on_the_packed_kernels(deg, precision, monkeypatch):
     monkeypatch.setenv("BN_PACKED", "0")
     y = precond(n, ia, ja, val, g, precision=precision)
     assert np.linalg.norm(x - y) <= TOL[precision] * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("nseg", [1, 3, 64, 593, 700])
+def test_segment_dots_of_uneven_segments(nseg):
+    """Slices per segment: 64 for one segment, 197 capped to 64 for three, 9 for
+    64, none (one slice) from 593 on; segments of 1 to 400 rows, so slices of no
+    row among them.  Every segment is a path graph with its own right-hand side."""
+    import scipy.sparse as sp
+    rng = np.random.default_rng(nseg)
+    sizes = rng.integers(1, 400 if nseg < 100 else 12, nseg)
+    sizes[0] = 1
+    blocks = [sp.diags([-np.ones(m - 1), np.full(m, 2.01), -np.ones(m - 1)], [-1, 0, 1])
+              for m in sizes]
+    A = sp.block_diag(blocks, format="csr")
+    A.sort_indices()
+    ptr = np.r_[0, np.cumsum(sizes)].astype(np.int32)
+    b = rng.standard_normal(A.shape[0])
+    s = amg.AMGSolver(A.shape[0], A.indptr, A.indices, A.data, min_size=50, stop=amg.STOP_RELRES)
+    x, its, rel, rc = s.solve_segmented(ptr, b, tol=1e-10)
+    s.close()
+    assert rc == 0 and (its > 0).all()
+    r = b - A @ x
+    for k in range(nseg):
+        q = slice(ptr[k], ptr[k + 1])
+        # the stopping test holds, and the reported residual is the true one
+        assert rel[k] < 1e-10
+        assert np.linalg.norm(r[q]) <= 1.01e-10 * np.linalg.norm(b[q])
