@@ -818,6 +818,7 @@ void IChol::load(CSR&& Lf, cudaStream_t s) {
 void IChol::finish(const int* aia, const int* aja, const double* aval, bool numeric,
                    cudaStream_t s) {
   const int g = grid_for(n, 256);
+  own_blocks = 0;
   Phase ph_lower("ichol lower", s);
   DBuf<int> flags(1, s);
   flags.zero();
@@ -915,10 +916,13 @@ void IChol::finish(const int* aia, const int* aja, const double* aval, bool nume
     bsrc.alloc((size_t)(fnnz > 0 ? fnnz : 1), s);
     BN_LAUNCH(k_bwd_fill, g, 256, 0, s, U.ia.p, U.ja.p, usrc.p, border.p, n, bia.p, bja.p, bsrc.p);
   }
-  // the tiled schedule serves the tiled single-vector form and the
-  // many-column sweeps of the block PCG
-  build_tiles(true, s);
-  build_tiles(false, s);
+  // the tiled schedule serves the tiled single-vector form and, where asked
+  // for, the many-column sweeps of the block PCG
+  const char* bt = getenv("BN_BLOCK_IC_TILES");
+  if (mode == kSweepTiles || (bt && atoi(bt))) {
+    build_tiles(true, s);
+    build_tiles(false, s);
+  }
   if (mode == kSweepSlab || mode == kSweepSlabW) {
     build_slab_partition(s);
     build_slab(true, s);
@@ -948,6 +952,11 @@ void IChol::remap(const int* inv, cudaStream_t s) {
   if (offd_nnz > 0) {
     BN_LAUNCH(k_map_ids, grid_for(offd_nnz, 256), 256, 0, s, fja.p, offd_nnz, inv, vfja.p);
     BN_LAUNCH(k_map_ids, grid_for(offd_nnz, 256), 256, 0, s, bja.p, offd_nnz, inv, vbja.p);
+  }
+  if (inv) {  // a solver's sweeps; a factor solved once does not repay the schedule
+    Phase ph("ichol owner form", s);
+    own_build(inv, s);
+    own_values(s);
   }
 }
 
@@ -985,6 +994,7 @@ void IChol::refresh_values() {
     slab_values(sf, s);
     slab_values(sb, s);
   }
+  own_values(s);
 }
 
 template <class T>
@@ -1172,6 +1182,12 @@ void IChol::solve(const T* b, T* y, T* x, cudaStream_t s) {
     BN_CUDA(cudaMemsetAsync(y, 0xFF, sizeof(T) * (size_t)n, s));
     run_tri_slab<T>(*this, true, b, y, x, wait.ctl(WT_IC_FWD), s);
     run_tri_slab<T>(*this, false, y, x, nullptr, wait.ctl(WT_IC_BWD), s);
+    return;
+  }
+  if (own_ready<T>()) {
+    BN_CUDA(cudaMemsetAsync(y, 0xFF, sizeof(T) * (size_t)n, s));
+    run_tri_own<T>(*this, true, b, y, x, wait.ctl(WT_IC_FWD), s);
+    run_tri_own<T>(*this, false, y, x, nullptr, wait.ctl(WT_IC_BWD), s);
     return;
   }
   if (mode == kSweepFlags || mode == kSweepSlab || mode == kSweepSlabW) {

@@ -14,6 +14,11 @@ template <class T>
 void run_tri_slab(const IChol& ic, bool forward, const T* in, T* out, T* clear, WaitCtl wc,
                   cudaStream_t s);
 
+// one sweep of the owner form (ic_own.cu); out pre-filled with the pending pattern
+template <class T>
+void run_tri_own(const IChol& ic, bool forward, const T* in, T* out, T* clear, WaitCtl wc,
+                 cudaStream_t s);
+
 struct IChol {
   struct Seg {
     int kind;    // 0: one wide level (grid launch); 1: run of narrow levels (one block)
@@ -96,6 +101,25 @@ struct IChol {
     return (mode == kSweepSlab || mode == kSweepSlabW) &&
            (sizeof(T) == 8 ? (sf.lead64 && sb.lead64) : (sf.lead32 && sb.lead32));
   }
+  // owner form (ic_own.cu), the sync-free sweep where it fits: per direction
+  // the rows in (owning block, level, index) order
+  struct Own {
+    DBuf<int> perm;               // position -> position in the level order
+    DBuf<int> step, base;         // first position of each step; of each block
+    DBuf<int2> range;             // per block: [first step, end step)
+    DBuf<int4> code;              // four dependencies per position
+    DBuf<int2> rec;               // {vector row, first further entry or -1}
+    DBuf<int> xcode;              // further entries, terminated per row
+    DBuf<double> val, diag, xval;
+    DBuf<float> val32, diag32, xval32;
+  };
+  Own of, ob;
+  DBuf<int> own_of;               // natural row -> block
+  int own_blocks = 0, own_rows = 0, own_limit = 0;  // blocks (0: not built), rows of the fullest
+  bool own_few = false;           // fewer blocks than SMs: smaller blocks
+  void own_build(const int* inv, cudaStream_t s);
+  void own_values(cudaStream_t s);
+  template <class T> bool own_ready() const;
   DBuf<int> fia, fja, fsrc; // forward rows (level order)
   DBuf<int> bia, bja, bsrc; // backward rows (reverse level order)
   // vector indices used by the solves: the rows/columns above mapped into

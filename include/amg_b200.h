@@ -214,7 +214,8 @@ typedef struct {
                            round trip per iteration); 0: host-driven loop */
   int ichol_form;       /* form of the fine IC(0) sweeps at the solver's precision:
                            0 level launches, 1 one cooperative launch, 2 sync-free
-                           32-row chunks, 3 tiles, 4 slabs (one block per SM) */
+                           (rows kept by their blocks, or 32-row chunks where they do
+                           not fit), 3 tiles, 4 slabs (one block per SM) */
 } amg_solve_stats;
 
 int amg_solver_stats(void* handle, amg_solve_stats* out);

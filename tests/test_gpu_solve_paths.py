@@ -57,3 +57,55 @@ def test_segment_dots_of_uneven_segments(nseg):
         # the stopping test holds, and the reported residual is the true one
         assert rel[k] < 1e-10
         assert np.linalg.norm(r[q]) <= 1.01e-10 * np.linalg.norm(b[q])
+
+
+def _random_spd(n, per_row, seed):
+    import scipy.sparse as sp
+    rng = np.random.default_rng(seed)
+    m = n * per_row // 2
+    u, v = rng.integers(0, n, m), rng.integers(0, n, m)
+    keep = u != v
+    w = sp.coo_matrix((rng.uniform(0.1, 1, keep.sum()), (u[keep], v[keep])), shape=(n, n))
+    w = (w + w.T).tocsr()
+    a = (sp.diags(np.asarray(w.sum(1)).ravel() + 0.1) - w).tocsr()
+    a.sort_indices()
+    return n, a.indptr.astype(np.int32), a.indices.astype(np.int32), a.data
+
+
+def _vascular(n, shuffle):
+    import scipy.sparse as sp
+    from blood_network_b200.network import vascular_network
+    net = vascular_network(depth=max(4, int(round(np.log2(0.2 * n)))), n_nodes=n, seed=5)
+    if not shuffle:
+        return net.n, net.indptr, net.indices, net.data
+    a = sp.csr_matrix((net.data, net.indices, net.indptr), shape=(net.n, net.n))
+    q = np.random.default_rng(9).permutation(net.n)
+    a = a[q][:, q].tocsr()
+    a.sort_indices()
+    return net.n, a.indptr.astype(np.int32), a.indices.astype(np.int32), a.data
+
+
+# one step; a last step of one row; rows of more than four entries; a row with
+# over a thousand; one block and several; a numbering that scatters every
+# dependency over the blocks; levels wide enough to be dealt
+OWN_CASES = {
+    "rows33": lambda: _random_spd(33, 4, 1),
+    "rows1025": lambda: _random_spd(1025, 3, 2),
+    "dense": lambda: _random_spd(900, 14, 3),
+    "hub": lambda: hub_matrix(side=40, hubs=(1200,), weak_hubs=(), seed=4),
+    "tree": lambda: _vascular(3_000, False),
+    "vascular": lambda: _vascular(60_000, False),
+    "shuffled": lambda: _vascular(60_000, True),
+}
+
+
+@pytest.mark.parametrize("precision", [amg.PREC_FP64, amg.PREC_MIXED])
+@pytest.mark.parametrize("name", sorted(OWN_CASES))
+def test_owner_sweeps_equal_the_chunked_ones(name, precision, monkeypatch):
+    n, ia, ja, val = OWN_CASES[name]()
+    g = np.random.default_rng(n).standard_normal(n)
+    kw = dict(precision=precision, min_size=30)
+    x = precond(n, ia, ja, val, g, **kw)
+    monkeypatch.setenv("BN_IC_OWN", "0")
+    y = precond(n, ia, ja, val, g, **kw)
+    assert x.tobytes() == y.tobytes() and np.isfinite(x).all()
