@@ -715,55 +715,6 @@ void jacobi_class(const DevMat<T>& A, const int* rows, int r0, int nr, const T* 
   BN_LAUNCH_PDL(k_scatter<T>, grid_for(nr, 256), 256, 0, s, rows, r0, nr, tmp, x);
 }
 
-// A whole sweep of a small level in one 1024-thread block: classes in
-// order (or reverse), a barrier between classes; overflow classes are
-// computed into tmp and copied back.  Warp per row.
-template <class T>
-__global__ void __launch_bounds__(1024)
-k_gs_level_block(const int* __restrict__ ia, const int* __restrict__ ja, const T* __restrict__ a,
-                 const int* __restrict__ cptr, const int* __restrict__ cjac, int ncls, int forward,
-                 const T* __restrict__ b, T* x, T* tmp) {
-  BN_PDL_ENTRY();
-  for (int q = 0; q < ncls; q++) {
-    const int c = forward ? q : ncls - 1 - q;
-    const int r0 = cptr[c], r1 = cptr[c + 1];
-    const bool jac = cjac[c] != 0;
-    const int lane = threadIdx.x & 31;
-    for (int i = r0 + (threadIdx.x >> 5); i < r1; i += (blockDim.x >> 5)) {
-      T sum = T(0), d = T(0);
-      int has = 0;
-      for (int k = ia[i] + lane; k < ia[i + 1]; k += 32) {
-        const int j = ja[k];
-        if (j == i) { d = a[k]; has = 1; }
-        else sum = dadd(sum, dmul(a[k], x[j]));
-      }
-      for (int off = 16; off > 0; off >>= 1) {
-        sum = dadd(sum, __shfl_xor_sync(0xffffffffu, sum, off));
-        const T od = __shfl_xor_sync(0xffffffffu, d, off);
-        const int oh = __shfl_xor_sync(0xffffffffu, has, off);
-        if (oh) { d = od; has = 1; }
-      }
-      if (lane == 0) {
-        const T xi = dsub(b[i], sum) / (has ? d : T(1));
-        if (jac) tmp[i - r0] = xi; else x[i] = xi;
-      }
-    }
-    __syncthreads();
-    if (jac) {
-      for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) x[i] = tmp[i - r0];
-      __syncthreads();
-    }
-  }
-}
-
-template <class T>
-void gs_level_block(const DevMat<T>& A, const int* cptr, const int* cjac, int ncls, bool forward,
-                    const T* b, T* x, T* tmp, cudaStream_t s) {
-  if (ncls <= 0) return;
-  BN_LAUNCH_PDL(k_gs_level_block<T>, 1, 1024, 0, s, A.ia, A.ja, A.val, cptr, cjac, ncls,
-            forward ? 1 : 0, b, x, tmp);
-}
-
 // out[t] = in[map[t]]  (gather) ; out[map[t]] = in[t]  (scatter)
 template <class T>
 __global__ void k_permute(const T* __restrict__ in, const int* __restrict__ map, int n,
@@ -1095,8 +1046,6 @@ void pcg_scalars(double* sc, int flexible, cudaStream_t s) {
   template void jacobi_class<T>(const DevMat<T>&, const int*, int, int, const T*, T*, T*, int,\
                                 cudaStream_t, int, const T*);                                \
   template void vpermute<T>(const T*, const int*, int, T*, bool, cudaStream_t);              \
-  template void gs_level_block<T>(const DevMat<T>&, const int*, const int*, int, bool,       \
-                                  const T*, T*, T*, cudaStream_t);                           \
   template void vzero<T>(T*, int, cudaStream_t);                                             \
   template void vadd<T>(const T*, const T*, int, T*, cudaStream_t);                          \
   template void dot_partials<T>(const T*, const T*, const T*, int, double*, double*,          \

@@ -85,10 +85,6 @@ void jacobi_class(const DevMat<T>& A, const int* rows, int r0, int nr, const T* 
 // x[r0 + t] = v[t], t < nr
 template <class T>
 void scatter_range(const T* v, int r0, int nr, T* x, cudaStream_t s);
-// all colour classes of a small level, one block, one launch
-template <class T>
-void gs_level_block(const DevMat<T>& A, const int* cptr, const int* cjac, int ncls, bool forward,
-                    const T* b, T* x, T* tmp, cudaStream_t s);
 // gather out[t] = in[map[t]] or scatter out[map[t]] = in[t]
 template <class T>
 void vpermute(const T* in, const int* map, int n, T* out, bool scatter, cudaStream_t s);

@@ -57,9 +57,17 @@ constexpr int kIrregularRow = 128;
 // packing (on the host) costs setup time: 80M entries as the line gained 0.7 %
 // on the 20M network's solve.
 constexpr long long kIrregularNnz = 8000000;
-constexpr int kSmallLevel = 2048;  // levels up to this size (without hub rows) sweep in one block
-// levels with at most this many entries take no split first sweep
+// levels with at most this many rows or entries take no split first sweep
+constexpr int kSmallLevel = 2048;
 constexpr long long kSmallLevelNnz = 65536;
+// Levels up to this many entries and rows, from the coarsest up, run as the
+// one-launch tail (vtail.cu): 16 SMs do an operation of a level in 2-4 us up to
+// here, less than the 4-5 us of a launch over all of them; beyond, the entries
+// count.  Whole solves, microseconds, without the tail / line at 65k / 140k /
+// 262k entries: 20k FP64 4438 / 3924 / 3851 / 3850, one preconditioner at 75k
+// 1033 / 971 / 945 / 1000, 64 packed networks 18134 / 16631 / 16980 / 16987.
+constexpr long long kTailNnz = 100000;
+constexpr int kTailRows = 32768;
 
 __global__ void k_color_round(const int* __restrict__ ia, const int* __restrict__ ja,
                               const int* __restrict__ set, int n, const int* __restrict__ color,
@@ -297,6 +305,146 @@ void Solver::drop_graphs() {
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   for (auto& g : loop)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+  tail64.ready = tail32.ready = false;
+}
+
+// First level of the tail: small levels only, all of them coloured, and a
+// program that fits its shared-memory copy.
+void Solver::choose_tail() {
+  const int nl = (int)lv.size();
+  tail_l0 = nl;
+  const char* e = getenv("BN_TAIL");  // 0: every level on launches of its own
+  if ((e && atoi(e) == 0) || nl < 2 || lv[nl - 1]->A.n > kTailDenseMax || lv[nl - 1]->A.n == 0) return;
+  if (opt.smoother != SMOOTHER_CF_GS && opt.smoother != SMOOTHER_GS) return;
+  if (!tail_nblk) tail_nblk = tail_cluster();
+  long long ops = 1;
+  for (int l = nl - 2; l >= 0; l--) {
+    const Level& L = *lv[l];
+    if (L.gs_rows.n == 0 || L.A.n == 0 || L.A.n > kTailRows || L.A.nnz > kTailNnz) break;
+    ops += 2 * ((long long)L.cptr.size() - 1) * opt.nu + 5;
+    if (ops > kTailMaxOps) break;
+    tail_l0 = l;
+  }
+}
+
+// The tail's programs in precision T (never inside a stream capture).
+template <class T>
+void Solver::ensure_tail() {
+  Tail<T>& P = tail<T>();
+  const int nl = (int)lv.size();
+  if (P.ready || tail_l0 >= nl) return;
+  constexpr bool f64 = sizeof(T) == 8;
+  auto vb = [&](int l) { return f64 ? (T*)lv[l]->b.p : (T*)lv[l]->b32.p; };
+  auto vx = [&](int l) { return f64 ? (T*)lv[l]->x.p : (T*)lv[l]->x32.p; };
+  auto vr = [&](int l) { return f64 ? (T*)lv[l]->r.p : (T*)lv[l]->r32.p; };
+  std::vector<TailOp<T>> ops;
+  std::vector<size_t> list_at;  // offset of an operation's row list
+  size_t list_n = 0;
+  // lanes per row: about the mean row length, as many as the cluster's
+  // threads give every row at once
+  auto lanes = [&](const CSR& M, int rows) {
+    int lg = 0;
+    while (lg < 5 && ((long long)M.n << lg) * 2 <= (long long)M.nnz + M.n &&
+           ((long long)rows << lg) * 2 <= (long long)kTailThreads * tail_nblk)
+      lg++;
+    return lg;
+  };
+  auto add = [&](int kind, int l, const CSR* M, const DBuf<float>* v32, int r0, int n, const T* b,
+                 const T* x, T* y, int top) {
+    TailOp<T> o{};
+    o.kind = kind;
+    o.lev = l;
+    o.r0 = r0;
+    o.n = n;
+    o.top = top;
+    if (M) {
+      o.lg = lanes(*M, n);
+      o.ia = M->ia.p;
+      o.ja = M->ja.p;
+      if constexpr (f64) o.a = M->val.p;
+      else o.a = v32->p;
+    }
+    if (l < nl - 1) {
+      if constexpr (f64) o.d = lv[l]->dg.p;
+      else o.d = lv[l]->dg32.p;
+    }
+    o.b = b;
+    o.x = x;
+    o.y = y;
+    list_at.push_back(M ? list_n : (size_t)-1);
+    if (M) list_n += n;
+    ops.push_back(o);
+  };
+  auto sweep = [&](int l, bool forward, bool zero) {
+    Level& L = *lv[l];
+    const int nc = (int)L.cptr.size() - 1;
+    int o0 = 0, on = 0;  // an overflow class just computed into r, not yet in x
+    for (int q = 0; q < nc; q++) {
+      const int c = forward ? q : nc - 1 - q;
+      const int r0 = L.cptr[c], n = L.cptr[c + 1] - r0;
+      const bool jac = L.cjac[c] && !zero;  // from zero every class reads earlier ones only
+      add(zero ? TK_GS0 : TK_GS, l, &L.Ap, &L.A32, r0, n, vb(l), vx(l), jac ? vr(l) : vx(l),
+          TT_B_IS_B | TT_X_IS_X | (jac ? 0 : TT_Y_IS_X));
+      ops.back().ov0 = o0;
+      ops.back().ovn = on;
+      ops.back().ov = vr(l);
+      o0 = r0;
+      on = jac ? n : 0;
+    }
+    if (on > 0) add(TK_COPY, l, nullptr, nullptr, o0, on, nullptr, vr(l), vx(l), TT_Y_IS_X);
+  };
+  const int nt = nl - tail_l0;
+  P.back.assign(nt, int2{0, 0});
+  P.fwd = P.sweep_f = P.sweep_b = P.back;
+  auto coarsest = [&]() {
+    add(TK_DENSE, nl - 1, nullptr, nullptr, 0, lv[nl - 1]->A.n, nullptr, vb(nl - 1), vx(nl - 1),
+        TT_X_IS_B | TT_Y_IS_X);
+    ops.back().dense = coarse.inv.p;
+  };
+  std::function<void(int)> back = [&](int l) {
+    P.back[l - tail_l0].x = (int)ops.size();
+    if (l == nl - 1) {
+      coarsest();
+    } else {
+      Level& L = *lv[l];
+      for (int k = 0; k < opt.nu; k++) sweep(l, true, k == 0);
+      add(TK_RES, l, &L.Ap, &L.A32, 0, L.A.n, vb(l), vx(l), vr(l), TT_B_IS_B | TT_X_IS_X);
+      add(TK_Y, l, &L.Rp, &L.R32, 0, L.Rp.n, nullptr, vr(l), vb(l + 1), 0);
+      back(l + 1);
+      add(TK_ADD, l, &L.Pp, &L.P32, 0, L.A.n, nullptr, vx(l + 1), vx(l), TT_Y_IS_X);
+    }
+    P.back[l - tail_l0].y = (int)ops.size();
+  };
+  std::function<void(int)> fwd = [&](int l) {
+    P.fwd[l - tail_l0].x = (int)ops.size();
+    if (l == nl - 1) {
+      coarsest();
+    } else {
+      Level& L = *lv[l];
+      add(TK_Y, l, &L.Rp, &L.R32, 0, L.Rp.n, nullptr, vb(l), vb(l + 1), TT_X_IS_B);
+      fwd(l + 1);
+      add(TK_Y, l, &L.Pp, &L.P32, 0, L.A.n, nullptr, vx(l + 1), vx(l), TT_Y_IS_X);
+      for (int k = 0; k < opt.nu; k++) sweep(l, false, false);
+    }
+    P.fwd[l - tail_l0].y = (int)ops.size();
+  };
+  back(tail_l0);
+  fwd(tail_l0);
+  for (int l = tail_l0; l < nl - 1; l++) {
+    P.sweep_f[l - tail_l0].x = (int)ops.size();
+    sweep(l, true, false);
+    P.sweep_f[l - tail_l0].y = P.sweep_b[l - tail_l0].x = (int)ops.size();
+    sweep(l, false, false);
+    P.sweep_b[l - tail_l0].y = (int)ops.size();
+  }
+  P.lists.alloc(list_n > 0 ? list_n : 1, s);
+  for (size_t q = 0; q < ops.size(); q++)
+    ops[q].list = list_at[q] == (size_t)-1 ? nullptr : P.lists.p + list_at[q];
+  P.ops.alloc(ops.size(), s);
+  P.ops.upload(ops.data(), ops.size());
+  tail_lists<T>(P.ops.p, (int)ops.size(), s);
+  BN_CUDA(cudaStreamSynchronize(s));  // ops is host memory
+  P.ready = true;
 }
 
 template <class T>
@@ -656,6 +804,7 @@ void permute_csr(const CSR& A, const int* perm, const int* cinv, CSR& B, cudaStr
 void Solver::build_solve_layout() {
   Phase ph("solve layout", s);
   const int nl = (int)lv.size();
+  choose_tail();
   auto coloured_level = [&](int l) {
     return l < nl - 1 && lv[l]->gs_rows.n > 0 &&
            (opt.smoother == SMOOTHER_CF_GS || opt.smoother == SMOOTHER_GS);
@@ -701,7 +850,10 @@ void Solver::build_solve_layout() {
         BN_LAUNCH(k_l1_diag, grid_for(L.A.n, 256), 256, 0, s, L.Ap.ia.p, L.Ap.val.p, L.A.n,
                   L.l1.p);
       }
-      if (use_packed) {  // packings only for the operators that run on them
+      // levels below the finest that run as the tail need no other layout
+      const bool in_tail = l > 0 && l >= tail_l0;
+      L.use_pkA = L.use_pkP = L.use_pkR = false;
+      if (use_packed && !in_tail) {  // packings only for the operators that run on them
         Phase ph2("packing", s, l);
         auto irregular = [](const RowLayout& lay, const CSR& M) {
           return lay.nlong > 0 || (lay.maxrow > kIrregularRow && M.nnz <= kIrregularNnz);
@@ -728,7 +880,7 @@ void Solver::build_solve_layout() {
       L.split = false;
       L.AL = CSR();
       L.AU = CSR();
-      if (coloured_level(l) && L.A.n > kSmallLevel && L.A.nnz > kSmallLevelNnz &&
+      if (coloured_level(l) && !in_tail && L.A.n > kSmallLevel && L.A.nnz > kSmallLevelNnz &&
           ((use_packed && L.use_pkA) || L.layA.nlong == 0)) {
         Phase ph3("split by class", s, l);
         build_split(L);
@@ -790,6 +942,7 @@ void Solver::alloc_vectors() {
 
 void Solver::prepare_f32() {
   const int nl = (int)lv.size();
+  tail32.ready = false;  // it holds the copies' addresses
   for (int l = 0; l < nl; l++) {
     Level& L = *lv[l];
     L.A32.alloc(L.Ap.nnz > 0 ? L.Ap.nnz : 1, s);
@@ -920,10 +1073,11 @@ void Solver::smooth(int l, const T* bb, T* xl, bool forward) {
       case SMOOTHER_GS: {
         const int nseg = (int)L.cptr.size() - 1;
         T* tmp = f64 ? (T*)L.r.p : (T*)L.r32.p;
-        // small levels sweep in one block, unless they hold hub rows (a warp
-        // per row would serialise a class behind them)
-        if (n <= kSmallLevel && L.layA.nlong == 0) {
-          gs_level_block<T>(A, L.d_cptr.p, L.d_cjac.p, nseg, forward, bb, xl, tmp, s);
+        if (l >= tail_l0) {  // a level of the tail: the sweep in one launch
+          ensure_tail<T>();
+          const Tail<T>& P = tail<T>();
+          const int2 q = forward ? P.sweep_f[l - tail_l0] : P.sweep_b[l - tail_l0];
+          tail_run<T>(P.ops.p, q.x, q.y, l, bb, xl, tail_nblk, s);
           break;
         }
         if (use_packed && L.use_pkA && L.pkG.ranges() == nseg) {
@@ -972,10 +1126,17 @@ void Solver::smooth(int l, const T* bb, T* xl, bool forward) {
   }
 }
 
-// backslash_rec (amg_cycle.c:180-212); xl is zero on entry
+// backslash_rec (amg_cycle.c:180-212); zero_guess: the initial guess is zero
+// (xl need not hold zeros), else xl
 template <class T>
 void Solver::backslash(int l, const T* bb, T* xl, bool zero_guess) {
   const int nl = (int)lv.size();
+  if (zero_guess && l >= tail_l0) {
+    ensure_tail<T>();
+    const int2 q = tail<T>().back[l - tail_l0];
+    tail_run<T>(tail<T>().ops.p, q.x, q.y, l, bb, xl, tail_nblk, s);
+    return;
+  }
   if (l == nl - 1) {
     coarse.apply<T>(bb, xl, s);
     return;
@@ -1008,6 +1169,7 @@ void Solver::backslash(int l, const T* bb, T* xl, bool zero_guess) {
       spmv<T>(SPMV_Y, mat<T>(L.AU, &L.AU32, &L.layAU), xl, nullptr, rr, s);
     }
   } else {
+    if (zero_guess) vzero<T>(xl, L.A.n, s);
     { Phase ph("gs forward", s, l); smooth<T>(l, bb, xl, true); }
     Phase ph("residual", s, l);
     if (use_packed && L.use_pkA)
@@ -1022,7 +1184,6 @@ void Solver::backslash(int l, const T* bb, T* xl, bool zero_guess) {
     else
       spmv<T>(SPMV_Y, mat<T>(L.Rp, &L.R32, &L.layR), rr, nullptr, cb, s);
   }
-  if (l + 1 < nl - 1) vzero<T>(cx, C.A.n, s);
   backslash<T>(l + 1, cb, cx, true);
   if (use_packed && L.use_pkP)  // x += P ec
     packed_apply<T>(PK_ADD, pmat<T>(L.Pp, L.P32, L.pkP), 0, cx, nullptr, xl, nullptr, 0, s);
@@ -1035,6 +1196,12 @@ void Solver::backslash(int l, const T* bb, T* xl, bool zero_guess) {
 template <class T>
 void Solver::fwdslash(int l, const T* bb, T* xl) {
   const int nl = (int)lv.size();
+  if (l >= tail_l0) {
+    ensure_tail<T>();
+    const int2 q = tail<T>().fwd[l - tail_l0];
+    tail_run<T>(tail<T>().ops.p, q.x, q.y, l, bb, xl, tail_nblk, s);
+    return;
+  }
   if (l == nl - 1) {
     coarse.apply<T>(bb, xl, s);
     return;
@@ -1070,7 +1237,6 @@ void Solver::precond_t(const T* g, T* out) {
   T* R2 = f64 ? (T*)r2.p : (T*)r2f.p;
   T* CO = f64 ? (T*)corr.p : (T*)corrf.p;
   DevMat<T> As = own_solve ? mat<T>(Aownp, &Aown32, &layOwn) : mat<T>(lv[0]->Ap, &lv[0]->A32, &lv[0]->layA);
-  vzero<T>(U1, n0, s);
   { Phase ph("backslash", s); backslash<T>(0, g, U1, true); }
   const bool fine_packed = use_packed && !own_solve && lv[0]->use_pkA && lv[0]->pkA.ranges() == 1;
   PackedMat<T> Ap0 = pmat<T>(lv[0]->Ap, lv[0]->A32, lv[0]->pkA);
@@ -1098,7 +1264,6 @@ void Solver::precond_t(const T* g, T* out) {
 // x += fwdslash(r), all on the hierarchy's level-0 operator, FP64
 void Solver::vcycle_apply(const double* g, double* out) {
   const int n0 = lv[0]->A.n;
-  vzero<double>(u1.p, n0, s);
   backslash<double>(0, g, u1.p, true);
   spmv<double>(SPMV_RES, mat<double>(lv[0]->Ap, nullptr, &lv[0]->layA), u1.p, g, r1.p, s);
   fwdslash<double>(0, r1.p, corr.p);
@@ -1153,6 +1318,8 @@ void l1_row_norms(const CSR& A, double* d_out, cudaStream_t s) {
 // z = M r for the PCG: r -> z (captured once per precision as a CUDA graph)
 void Solver::precond(const double* g, double* out) {
   const int mode = opt.precision == AMG_PREC_MIXED ? 1 : 0;
+  if (mode == 1) ensure_tail<float>();  // before any capture
+  else ensure_tail<double>();
   const bool use_graph = (g == r.p && out == z.p) && !trace_on() && !capture_direct;
   if (use_graph && graph[mode]) {
     BN_CUDA(cudaGraphLaunch(graph[mode], s));

@@ -6,6 +6,7 @@
 #include "dense.cuh"
 #include "solve_kernels.cuh"
 #include "packed.cuh"
+#include "vtail.cuh"
 #include "../../include/amg_b200.h"
 
 #include <cstdlib>
@@ -65,6 +66,16 @@ struct Level {
   DBuf<float> b32, x32, r32;
 };
 
+// The coarse tail's operations (vtail.cuh) and, per level of the tail, the
+// ranges of its backslash, its fwdslash and one forward / backward sweep.
+template <class T>
+struct Tail {
+  bool ready = false;
+  DBuf<TailOp<T>> ops;
+  DBuf<int4> lists;
+  std::vector<int2> back, fwd, sweep_f, sweep_b;  // indexed by level - first
+};
+
 struct BlockWork;  // work vectors of a many-right-hand-side solve (block.cu)
 
 struct Solver {
@@ -120,6 +131,18 @@ struct Solver {
   const RowLayout& lay_solve() const { return own_solve ? layOwn : lv[0]->layA; }
   const CSR& Asolve_p() const { return own_solve ? Aownp : lv[0]->Ap; }
   void build_solve_layout();
+  // The coarse tail: levels tail_l0 .. coarsest (tail_l0 = number of levels:
+  // none).  Its programs hold the vectors' addresses, so they go with the
+  // graphs (drop_graphs) and are made again before the next use.
+  int tail_l0 = 0, tail_nblk = 0;
+  Tail<double> tail64;
+  Tail<float> tail32;
+  template <class T> Tail<T>& tail() {
+    if constexpr (sizeof(T) == 8) return tail64;
+    else return tail32;
+  }
+  void choose_tail();
+  template <class T> void ensure_tail();
   template <class T> void smooth(int l, const T* bb, T* xl, bool forward);
   // zero_guess: xl holds zeros on entry (every call inside the
   // preconditioner), which allows the split first sweep

@@ -109,3 +109,62 @@ def test_owner_sweeps_equal_the_chunked_ones(name, precision, monkeypatch):
     monkeypatch.setenv("BN_IC_OWN", "0")
     y = precond(n, ia, ja, val, g, **kw)
     assert x.tobytes() == y.tobytes() and np.isfinite(x).all()
+
+
+# levels that are all the tail, partly, and with rows taken by a lane group, a
+# warp (over 8 entries a lane) and a block (over 256 entries); several sweeps;
+# plain Gauss-Seidel order; HMIS hierarchies
+TAIL_CASES = {
+    "one level": (lambda: _random_spd(200, 4, 6), dict(min_size=500)),
+    "two levels": (lambda: _random_spd(601, 4, 7), dict(min_size=500)),
+    "vascular 2k": (lambda: _vascular(2_000, False), {}),
+    "vascular 60k": (lambda: _vascular(60_000, False), {}),
+    "hmis": (lambda: _vascular(20_000, False), dict(coarsening=amg.COARSEN_HMIS, threshold=0.5)),
+    "hubs": (lambda: hub_matrix(side=50, hubs=(60, 255, 256, 257, 1100, 2300), weak_hubs=(),
+                                seed=8), {}),
+    "two sweeps": (lambda: _vascular(5_000, False), dict(nu=2)),
+    "plain order": (lambda: _vascular(5_000, False), dict(smoother=amg.SMOOTHER_GS)),
+}
+
+
+@pytest.mark.parametrize("precision", [amg.PREC_FP64, amg.PREC_MIXED])
+@pytest.mark.parametrize("name", sorted(TAIL_CASES))
+def test_tail_equals_the_level_launches(name, precision, monkeypatch):
+    make, kw = TAIL_CASES[name]
+    n, ia, ja, val = make()
+    g = np.random.default_rng(n).standard_normal(n)
+    x = precond(n, ia, ja, val, g, precision=precision, **kw)
+    monkeypatch.setenv("BN_TAIL", "0")
+    y = precond(n, ia, ja, val, g, precision=precision, **kw)
+    assert np.linalg.norm(x - y) <= TOL[precision] * np.linalg.norm(y)
+
+
+def test_tail_after_the_hierarchy_changes(monkeypatch):
+    """A new smoother, precision and new values rebuild the tail's programs."""
+    n, ia, ja, val = _vascular(4_000, False)
+    g = np.random.default_rng(2).standard_normal(n)
+
+    def passes():
+        s = amg.AMGSolver(n, ia, ja, val, min_size=200)
+        out = [s.precond(g)]
+        s.set_smoother(amg.SMOOTHER_GS)
+        out.append(s.precond(g))
+        s.set_smoother(amg.SMOOTHER_JACOBI, 0.6)
+        out.append(s.precond(g))
+        s.set_smoother(amg.SMOOTHER_CF_GS)
+        out.append(s.precond(g))
+        s.set_precision(amg.PREC_MIXED)
+        out.append(s.precond(g))
+        s.set_precision(amg.PREC_FP64)
+        s.update(ia, ja, 2.0 * val)
+        out.append(s.precond(g))
+        s.close()
+        return out
+
+    tail = passes()
+    monkeypatch.setenv("BN_TAIL", "0")
+    plain = passes()
+    assert tail[0].tobytes() == tail[3].tobytes() and tail[0].tobytes() != tail[1].tobytes()
+    for k, (x, y) in enumerate(zip(tail, plain)):
+        tol = TOL[amg.PREC_MIXED if k == 4 else amg.PREC_FP64]
+        assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y), k
