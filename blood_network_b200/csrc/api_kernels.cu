@@ -57,7 +57,9 @@ static void coarsen_api(const dcsr_mat* S, int method, int max_lam, int* cf, int
     CSR d;
     to_device(S, d, s, false);
     DBuf<int> dcf(S->row > 0 ? S->row : 1, s);
-    int nc = coarsen(d, method, max_lam, dcf.p, s);
+    RandDraws draws;
+    int nc = coarsen(d, method, max_lam, dcf.p, s, draws);
+    if (method == COARSEN_PMIS && d.n > 0) pmis_rand_state(d.n);
     dcf.download(cf, S->row);
     BN_CUDA(cudaStreamSynchronize(s));
     *n_coarse = nc;

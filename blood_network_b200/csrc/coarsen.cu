@@ -421,7 +421,33 @@ static int count_c(const int* cf, int n, cudaStream_t s) {
   return read_scalar(c.p, s);
 }
 
-int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s) {
+// The first n draws after srand(12345).  Every level of a hierarchy starts the
+// sequence again, so the levels share the finest one's draws (a level of its
+// own drawing and uploading from the host took 15 ms of a 1M-row PMIS level,
+// 27 ms over the hierarchy; here 5.3).  Device draws pay from some ten
+// thousand points on: the jump matrices cost the host half a millisecond.
+constexpr int kHostDraws = 32768;
+const int* RandDraws::first(int n, bool host_ok, cudaStream_t s) {
+  if ((size_t)n <= d.n) return d.p;
+  d.alloc(n, s);
+  if (host_ok && n <= kHostDraws) {
+    std::vector<int> h(n);
+    srand(12345);
+    for (int i = 0; i < n; i++) h[i] = rand();
+    d.upload(h.data(), n);
+    BN_CUDA(cudaStreamSynchronize(s));  // h must outlive the copy
+  } else {
+    crand_device(12345u, d.p, n, s);
+  }
+  return d.p;
+}
+
+void pmis_rand_state(int n) {
+  srand(12345);
+  for (int i = 0; i < n; i++) rand();
+}
+
+int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s, RandDraws& draws) {
   (void)max_lam;
   const int n = S.n;
   if (n == 0) return 0;
@@ -444,14 +470,10 @@ int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s) {
   const int glong = nlong < 4096 ? nlong : 4096;
 
   if (method == COARSEN_PMIS) {
-    // rand() sequence after srand(12345), drawn from the host C library
-    std::vector<int> h(n);
-    srand(12345);
-    for (int i = 0; i < n; i++) h[i] = rand();
-    DBuf<int> rnd(n, s);
-    rnd.upload(h.data(), n);
-    BN_LAUNCH(k_pmis_weights, g, 256, 0, s, lam.p, rnd.p, n, w.p, cf);
-    BN_CUDA(cudaStreamSynchronize(s));  // h must outlive the copy
+    // rand() sequence after srand(12345) (the caller sets the C library's own
+    // state, pmis_rand_state)
+    const int* rnd = draws.first(n, true, s);
+    BN_LAUNCH(k_pmis_weights, g, 256, 0, s, lam.p, rnd, n, w.p, cf);
     long long undecided = n;
     for (long long round = 0; undecided > 0 && round <= n; round++) {
       ctr.zero();
@@ -474,7 +496,6 @@ int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s) {
     // RS measure: lambda_i = |S^T_i|; the classical RS routine leaves
     // lambda_0 at zero (rs_classical.c:118-123), reproduced here.
     if (method == COARSEN_RS) BN_CUDA(cudaMemsetAsync(lam.p, 0, sizeof(int), s));
-    DBuf<int> rnd;
     if (method == COARSEN_HMIS) {
       // ties between equal measures: the reference HMIS's weights
       // lambda_i + rand()/RAND_MAX after srand(12345) (rs_classical.c:
@@ -483,9 +504,8 @@ int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s) {
       // device in chunks from jump-ahead windows), so the
       // caller's rand() state is left alone as the reference's first pass
       // leaves it.
-      rnd.alloc(n, s);
-      crand_device(12345u, rnd.p, n, s);
-      BN_LAUNCH(k_pmis_weights, g, 256, 0, s, lam.p, rnd.p, n, w.p, cf);
+      const int* rnd = draws.first(n, false, s);
+      BN_LAUNCH(k_pmis_weights, g, 256, 0, s, lam.p, rnd, n, w.p, cf);
     } else {
       BN_LAUNCH(k_rs_measure, g, 256, 0, s, lam.p, n, w.p);
     }

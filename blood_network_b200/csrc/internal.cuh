@@ -18,7 +18,17 @@ void strength(const CSR& A, double theta, CSR& S, int* max_lam, cudaStream_t s);
 // ---- coarsen.cu
 enum Coarsening : int { COARSEN_RS = 0, COARSEN_PMIS = 1, COARSEN_HMIS = 2 };
 // cf[i] = +1 (C) / -1 (F); returns the number of C points.
-int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s);
+// rand() draws after srand(12345) on the device, kept for the levels of one
+// hierarchy.  host_ok: short sequences may come from the C library itself
+// (which moves its state).
+struct RandDraws {
+  DBuf<int> d;
+  const int* first(int n, bool host_ok, cudaStream_t s);
+};
+int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s, RandDraws& draws);
+// The C library's rand() state as the reference's PMIS of n points leaves it
+// (rs_classical.c:246-371: srand(12345), n draws).
+void pmis_rand_state(int n);
 
 // ---- interp.cu
 void interpolation(const CSR& A, const CSR& S, const int* cf, int n_coarse, CSR& P,

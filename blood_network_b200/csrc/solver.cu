@@ -1008,6 +1008,8 @@ void Solver::build(CSR&& A0) {
   lv[0]->A = std::move(A0);
   const int max_levels =
       (opt.max_levels > 0 && opt.max_levels <= AMG_MAX_LEVELS) ? opt.max_levels : AMG_MAX_LEVELS;
+  RandDraws draws;
+  int pmis_points = 0;
   while (lv.back()->A.n >= opt.min_size && (int)lv.size() < max_levels) {
     Level& cur = *lv.back();
     const int nf = cur.A.n;
@@ -1015,7 +1017,8 @@ void Solver::build(CSR&& A0) {
     { Phase ph("strength", s, li); strength(cur.A, opt.threshold, cur.S, &cur.max_lam, s); }
     cur.cf.alloc(nf, s);
     int nc;
-    { Phase ph("coarsen", s, li); nc = coarsen(cur.S, opt.coarsening, cur.max_lam, cur.cf.p, s); }
+    { Phase ph("coarsen", s, li); nc = coarsen(cur.S, opt.coarsening, cur.max_lam, cur.cf.p, s, draws); }
+    if (opt.coarsening == COARSEN_PMIS) pmis_points = nf;
     cur.n_coarse = nc;
     if (nc == 0 || nc >= nf) break;  // coarsening stalled (:78-83)
     { Phase ph("interpolation", s, li); interpolation(cur.A, cur.S, cur.cf.p, nc, cur.P, s); }
@@ -1026,6 +1029,7 @@ void Solver::build(CSR&& A0) {
     lv.emplace_back(new Level());
     lv.back()->A = std::move(Acs);
   }
+  if (pmis_points > 0) pmis_rand_state(pmis_points);  // as its last call leaves it
   finish_setup();
   cudaEventRecord(ev1, s);
   BN_CUDA(cudaEventSynchronize(ev1));
