@@ -138,17 +138,196 @@ __device__ __forceinline__ int hub_find(const int* __restrict__ keys, const int*
 // denominator in that order; each slot of P's row receives its terms in the
 // same sequence as in the thread kernel.
 constexpr int kWarpRow = 32;
+// ... and so are shorter ones whose strong F neighbours' rows hold more than
+// kWarpWalk entries together: a thread walks them twice, a slot search per
+// entry, and a few such rows were the whole time of a call on a coarse level
+// (150k-row network: 0.96 ms a call over the levels, now 0.15).
+constexpr int kWarpWalk = 96;
 
 __device__ __forceinline__ bool warp_row(const int* __restrict__ aia, const int* __restrict__ sia,
+                                         const int* __restrict__ sja, const int* __restrict__ cf,
                                          int i) {
-  return aia[i + 1] - aia[i] > kWarpRow && sia[i + 1] - sia[i] <= kInterpMaxC;
+  const int s0 = sia[i], s1 = sia[i + 1];
+  if (s1 - s0 > kInterpMaxC) return false;
+  if (aia[i + 1] - aia[i] > kWarpRow) return true;
+  int walk = 0;
+  for (int k = s0; k < s1; k++) {
+    const int j = sja[k];
+    if (cf[j] != 1) walk += aia[j + 1] - aia[j];
+  }
+  return walk > kWarpWalk;
 }
 
-__global__ void k_warp_rows(const int* __restrict__ aia, const int* __restrict__ sia,
-                            const int* __restrict__ cf, int n, int* __restrict__ list,
+// F rows with more strong points than a warp takes, up to kBlockMaxS: a block each
+constexpr int kBlockMaxS = 2048;
+__device__ __forceinline__ bool block_row(const int* __restrict__ sia, int i) {
+  const int ns = sia[i + 1] - sia[i];
+  return ns > kInterpMaxC && ns <= kBlockMaxS;
+}
+
+// wide[i] = 1 for rows left to the warp or block kernel; counter[0] warp rows,
+// from the front of list; counter[1] block rows, from the back
+__global__ void k_wide_rows(const int* __restrict__ aia, const int* __restrict__ sia,
+                            const int* __restrict__ sja, const int* __restrict__ cf, int n,
+                            unsigned char* __restrict__ wide, int* __restrict__ list,
                             int* counter) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if (cf[i] != 1 && warp_row(aia, sia, i)) list[atomicAdd(counter, 1)] = i;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const bool f = cf[i] != 1;
+    const bool blk = f && block_row(sia, i), wrp = f && !blk && warp_row(aia, sia, sja, cf, i);
+    wide[i] = blk || wrp;
+    if (wrp) list[atomicAdd(counter, 1)] = i;
+    if (blk) list[n - 1 - atomicAdd(counter + 1, 1)] = i;
+  }
+}
+
+// An F row with many strong points, a block each.  One thread per row found each
+// entry's slot by walking S_i (1.0-2.7 ms a call on levels with rows of some
+// hundred strong points, all of it one thread); here S_i sits in a
+// shared-memory hash (column -> slot among the C points, or F), the entries of
+// A_i are classified by all threads, the strong F neighbours' denominators are
+// formed by a warp each and the terms are then added neighbour by neighbour.
+// The operations and their order are the thread kernel's: the weak entries
+// are added in row order by one thread, each denominator in row order, each
+// slot's terms in the order of the neighbours in A_i.
+constexpr int kBlkThreads = 256, kBlkTable = 2 * kBlockMaxS;
+struct InterpBlock {
+  int key[kBlkTable];      // column, -1 empty
+  int slot[kBlkTable];     // C: rank among the C points of S_i; F: -1
+  int fk[kBlockMaxS];      // entries of A_i that are strong F points, in order
+  double den[kBlockMaxS];  // their denominators
+  double num[kBlockMaxS];  // the row of P by slot
+  double weak[kBlkThreads];
+};
+__device__ __forceinline__ int blk_find(const InterpBlock& t, int m, bool* in) {
+  int at = (int)(hub_hash(m) >> 20) & (kBlkTable - 1);
+  while (true) {
+    const int k = t.key[at];
+    if (k == m) { *in = true; return t.slot[at]; }
+    if (k == -1) { *in = false; return -1; }
+    at = (at + 1) & (kBlkTable - 1);
+  }
+}
+// inclusive rank of the threads with flag set, in thread order, plus the block's total
+__device__ __forceinline__ int blk_rank(bool flag, int* wsum, int* total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned b = __ballot_sync(0xffffffffu, flag);
+  if (lane == 0) wsum[w] = __popc(b);
+  __syncthreads();
+  int before = 0, all = 0;
+  for (int q = 0; q < kBlkThreads / 32; q++) {
+    before += q < w ? wsum[q] : 0;
+    all += wsum[q];
+  }
+  __syncthreads();
+  *total = all;
+  return before + __popc(b & ((1u << lane) - 1u));
+}
+
+__global__ void __launch_bounds__(kBlkThreads)
+k_interp_values_block(const int* __restrict__ aia, const int* __restrict__ aja,
+                      const double* __restrict__ aval, const int* __restrict__ sia,
+                      const int* __restrict__ sja, const int* __restrict__ cf,
+                      const int* __restrict__ rows, const int* __restrict__ pia,
+                      double* __restrict__ pval) {
+  extern __shared__ __align__(16) unsigned char blk_mem[];
+  InterpBlock& t = *reinterpret_cast<InterpBlock*>(blk_mem);
+  __shared__ int wsum[kBlkThreads / 32];
+  __shared__ double s_diag, s_hat;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int i = rows[blockIdx.x];
+  const int s0 = sia[i], ns = sia[i + 1] - s0, a0 = aia[i], a1 = aia[i + 1], p0 = pia[i];
+  for (int q = tid; q < kBlkTable; q += kBlkThreads) t.key[q] = -1;
+  if (tid == 0) s_diag = 0.0;
+  __syncthreads();
+  int nc = 0;
+  for (int base = 0; base < ns; base += kBlkThreads) {
+    const int q = base + tid;
+    int m = -1, kind = 0;
+    if (q < ns) {
+      m = sja[s0 + q];
+      kind = cf[m];
+    }
+    int total;
+    const int r = nc + blk_rank(kind == 1, wsum, &total);
+    if (kind == 1) t.num[r] = 0.0;
+    if (kind == 1 || kind == -1) {
+      int at = (int)(hub_hash(m) >> 20) & (kBlkTable - 1);
+      while (atomicCAS(&t.key[at], -1, m) != -1) at = (at + 1) & (kBlkTable - 1);
+      t.slot[at] = kind == 1 ? r : -1;
+    }
+    nc += total;
+  }
+  __syncthreads();
+  // A_i: diagonal, direct C terms, weak sum, the strong F entries
+  double weak = 0.0;
+  int nf = 0;
+  for (int base = a0; base < a1; base += kBlkThreads) {
+    const int k = base + tid;
+    bool is_weak = false, is_f = false;
+    double a = 0.0;
+    if (k < a1) {
+      const int j = aja[k];
+      a = aval[k];
+      if (j == i) {
+        s_diag = a;
+      } else {
+        bool in;
+        const int sl = blk_find(t, j, &in);
+        if (!in) is_weak = true;
+        else if (sl >= 0) t.num[sl] = xadd(t.num[sl], a);  // one entry per column
+        else is_f = true;
+      }
+    }
+    int nw, nn;
+    const int rw = blk_rank(is_weak, wsum, &nw);
+    if (is_weak) t.weak[rw] = a;
+    const int rf = blk_rank(is_f, wsum, &nn);
+    if (is_f) t.fk[nf + rf] = k;
+    nf += nn;
+    __syncthreads();
+    if (tid == 0)
+      for (int q = 0; q < nw; q++) weak = xadd(weak, t.weak[q]);
+    __syncthreads();
+  }
+  // denominators: a warp per neighbour, the entries in C_i added in row order
+  for (int f = w; f < nf; f += kBlkThreads / 32) {
+    const int kk = aja[t.fk[f]];
+    double den = 0.0;
+    for (int base = aia[kk]; base < aia[kk + 1]; base += 32) {
+      const int l = base + lane;
+      bool hit = false;
+      double a = 0.0;
+      if (l < aia[kk + 1]) {
+        bool in;
+        hit = blk_find(t, aja[l], &in) >= 0;
+        if (hit) a = aval[l];
+      }
+      for (unsigned m = __ballot_sync(0xffffffffu, hit); m; m &= m - 1)
+        den = xadd(den, __shfl_sync(0xffffffffu, a, __ffs(m) - 1));
+    }
+    if (lane == 0) t.den[f] = den;
+  }
+  __syncthreads();
+  double hat = xadd(s_diag, weak);  // of thread 0
+  for (int f = 0; f < nf; f++) {
+    const int ke = t.fk[f], kk = aja[ke];
+    const double a_ik = aval[ke], den = t.den[f];
+    if (fabs(den) < 1e-15) {
+      hat = xadd(hat, a_ik);
+      continue;
+    }
+    for (int l = aia[kk] + tid; l < aia[kk + 1]; l += kBlkThreads) {
+      bool in;
+      const int sl = blk_find(t, aja[l], &in);
+      if (sl >= 0) t.num[sl] = xadd(t.num[sl], xdiv(xmul(a_ik, aval[l]), den));
+    }
+    __syncthreads();
+  }
+  if (tid == 0) s_hat = hat;
+  __syncthreads();
+  const bool div = fabs(s_hat) > 1e-15;
+  const double nd = -s_hat;
+  for (int q = tid; q < nc; q += kBlkThreads) pval[p0 + q] = div ? xdiv(t.num[q], nd) : t.num[q];
 }
 
 constexpr int kInterpWarps = 4;
@@ -291,6 +470,7 @@ k_interp_values_warp(const int* __restrict__ aia, const int* __restrict__ aja,
 __global__ void k_interp_values(const int* __restrict__ aia, const int* __restrict__ aja,
                                 const double* __restrict__ aval, const int* __restrict__ sia,
                                 const int* __restrict__ sja, const int* __restrict__ cf, int n,
+                                const unsigned char* __restrict__ wide,
                                 const int* __restrict__ pia, double* __restrict__ pval,
                                 const int* __restrict__ hubidx, const int* __restrict__ hoff,
                                 const int* __restrict__ hkeys, const int* __restrict__ hvals) {
@@ -300,7 +480,7 @@ __global__ void k_interp_values(const int* __restrict__ aia, const int* __restri
       pval[p0] = 1.0;
       continue;
     }
-    if (warp_row(aia, sia, i)) continue;  // k_interp_values_warp
+    if (wide[i]) continue;  // the kernels above
     const int s0 = sia[i], s1 = sia[i + 1];
     for (int p = p0; p < p1; p++) pval[p] = 0.0;
     double diag = 0.0, weak = 0.0;
@@ -397,7 +577,7 @@ __global__ void k_interp_values(const int* __restrict__ aia, const int* __restri
 void interpolation_values(const CSR& A, const CSR& S, const int* cf, CSR& P, cudaStream_t s) {
   if (A.n == 0) return;
   const int n = A.n;
-  DBuf<int> hubidx(n, s), hubrows(n, s), ctr(1, s);
+  DBuf<int> hubidx(n, s), hubrows(n, s), ctr(2, s);
   ctr.zero();
   BN_LAUNCH(k_hub_mark, grid_for(n, 256), 256, 0, s, A.ia.p, n, hubidx.p, hubrows.p, ctr.p);
   const int nh = read_scalar(ctr.p, s);
@@ -411,12 +591,23 @@ void interpolation_values(const CSR& A, const CSR& S, const int* cf, CSR& P, cud
     keys.fill_bytes(0xff);
     BN_LAUNCH(k_hub_fill, nh, 256, 0, s, A.ia.p, A.ja.p, hubrows.p, hoff.p, keys.p, vals.p);
   }
-  BN_LAUNCH(k_interp_values, grid_for(n, 128), 128, 0, s, A.ia.p, A.ja.p, A.val.p, S.ia.p,
-            S.ja.p, cf, n, P.ia.p, P.val.p, nh > 0 ? hubidx.p : nullptr, hoff.p, keys.p,
-            vals.p);
+  DBuf<unsigned char> wide(n, s);
   ctr.zero();
-  BN_LAUNCH(k_warp_rows, grid_for(n, 256), 256, 0, s, A.ia.p, S.ia.p, cf, n, hubrows.p, ctr.p);
-  const int nw = read_scalar(ctr.p, s);
+  BN_LAUNCH(k_wide_rows, grid_for(n, 256), 256, 0, s, A.ia.p, S.ia.p, S.ja.p, cf, n, wide.p,
+            hubrows.p, ctr.p);
+  BN_LAUNCH(k_interp_values, grid_for(n, 128), 128, 0, s, A.ia.p, A.ja.p, A.val.p, S.ia.p,
+            S.ja.p, cf, n, wide.p, P.ia.p, P.val.p, nh > 0 ? hubidx.p : nullptr, hoff.p, keys.p,
+            vals.p);
+  int hn[2];
+  ctr.download(hn, 2);
+  BN_CUDA(cudaStreamSynchronize(s));
+  const int nw = hn[0];
+  if (hn[1] > 0) {
+    BN_CUDA(cudaFuncSetAttribute(k_interp_values_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(InterpBlock)));
+    BN_LAUNCH(k_interp_values_block, hn[1], kBlkThreads, sizeof(InterpBlock), s, A.ia.p, A.ja.p,
+              A.val.p, S.ia.p, S.ja.p, cf, hubrows.p + (n - hn[1]), P.ia.p, P.val.p);
+  }
   if (nw > 0)
     BN_LAUNCH(k_interp_values_warp, grid_for((long long)nw * 32, 32 * kInterpWarps, 8),
               32 * kInterpWarps, 0, s, A.ia.p, A.ja.p, A.val.p, S.ia.p, S.ja.p, S.val.p, cf,
