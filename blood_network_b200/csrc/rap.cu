@@ -301,35 +301,72 @@ k_rap_count_warp(const int* __restrict__ ria, const int* __restrict__ rja,
   }
 }
 
-__global__ void __launch_bounds__(32)
+// The rows with many products, a block each: a count does not depend on the order
+// of the insertions, so all threads share the row's table.  With a warp per row
+// the launch waited for its longest row (levels of a 1M-row network: 660 us a
+// call, now 294; the one with rows beyond shared tables 2,100 -> 680).
+constexpr int kCountThreads = 256;
+__device__ int rap_count_block(int ic, Table t, const int* __restrict__ ria,
+                               const int* __restrict__ rja, const int* __restrict__ aia,
+                               const int* __restrict__ aja, const int* __restrict__ pia,
+                               const int* __restrict__ pja) {
+  __shared__ int total;
+  const int tid = threadIdx.x;
+  for (unsigned q = tid; q <= t.mask; q += kCountThreads) t.keys[q] = -1;
+  if (tid == 0) total = 0;
+  __syncthreads();
+  int cnt = 0;
+  if (tid == 0) cnt += table_insert_atomic(t, ic);
+  const int lane = tid & 31, w = tid >> 5;
+  auto entry = [&](int k2) {
+    const int i2 = aja[k2];
+    for (int k3 = pia[i2]; k3 < pia[i2 + 1]; k3++) cnt += table_insert_atomic(t, pja[k3]);
+  };
+  // R's entries a warp each; rows of A that are long themselves take the block
+  for (int k1 = ria[ic] + w; k1 < ria[ic + 1]; k1 += kCountThreads / 32) {
+    const int i1 = rja[k1], a0 = aia[i1], a1 = aia[i1 + 1];
+    if (a1 - a0 > kCountThreads) continue;
+    for (int k2 = a0 + lane; k2 < a1; k2 += 32) entry(k2);
+  }
+  for (int k1 = ria[ic]; k1 < ria[ic + 1]; k1++) {
+    const int i1 = rja[k1], a0 = aia[i1], a1 = aia[i1 + 1];
+    if (a1 - a0 <= kCountThreads) continue;
+    for (int k2 = a0 + tid; k2 < a1; k2 += kCountThreads) entry(k2);
+  }
+  for (int off = 16; off > 0; off >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
+  if ((tid & 31) == 0) atomicAdd(&total, cnt);
+  __syncthreads();
+  const int c = total;
+  __syncthreads();
+  return c;
+}
+
+__global__ void __launch_bounds__(kCountThreads)
 k_rap_count_big(const int* __restrict__ ria, const int* __restrict__ rja,
                 const int* __restrict__ aia, const int* __restrict__ aja,
                 const int* __restrict__ pia, const int* __restrict__ pja,
                 const int* __restrict__ rows, int m, int* __restrict__ cnt_out) {
   extern __shared__ int dyn[];
-  const int lane = threadIdx.x & 31;
   Table t{dyn, nullptr, nullptr, kBigCap - 1};
   for (int q = blockIdx.x; q < m; q += gridDim.x) {
     const int ic = rows[q];
-    int c = rap_count_row(ic, t, lane, ria, rja, aia, aja, pia, pja);
-    if (lane == 0) cnt_out[ic] = c;
+    const int c = rap_count_block(ic, t, ria, rja, aia, aja, pia, pja);
+    if (threadIdx.x == 0) cnt_out[ic] = c;
   }
 }
 
-__global__ void k_rap_count_huge(const int* __restrict__ ria, const int* __restrict__ rja,
-                                 const int* __restrict__ aia, const int* __restrict__ aja,
-                                 const int* __restrict__ pia, const int* __restrict__ pja,
-                                 const int* __restrict__ rows, int m,
-                                 const long long* __restrict__ toff, int* __restrict__ gkeys,
-                                 int* __restrict__ cnt_out) {
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < m; q += warps) {
+__global__ void __launch_bounds__(kCountThreads)
+k_rap_count_huge(const int* __restrict__ ria, const int* __restrict__ rja,
+                 const int* __restrict__ aia, const int* __restrict__ aja,
+                 const int* __restrict__ pia, const int* __restrict__ pja,
+                 const int* __restrict__ rows, int m, const long long* __restrict__ toff,
+                 int* __restrict__ gkeys, int* __restrict__ cnt_out) {
+  for (int q = blockIdx.x; q < m; q += gridDim.x) {
     const int ic = rows[q];
     const long long off = toff[q];
     Table t{gkeys + off, nullptr, nullptr, (unsigned)(toff[q + 1] - off) - 1};
-    int c = rap_count_row(ic, t, lane, ria, rja, aia, aja, pia, pja);
-    if (lane == 0) cnt_out[ic] = c;
+    const int c = rap_count_block(ic, t, ria, rja, aia, aja, pia, pja);
+    if (threadIdx.x == 0) cnt_out[ic] = c;
   }
 }
 
@@ -937,7 +974,7 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
       BN_LAUNCH(k_rap_count_warp, grid_for(rc.count[0], kRapWarps, 64), 32 * kRapWarps, 0, s,
                 R.ia.p, R.ja.p, A.ia.p, A.ja.p, P.ia.p, P.ja.p, L0, rc.count[0], cnt.p);
     if (rc.count[1])
-      BN_LAUNCH(k_rap_count_big, grid_for(rc.count[1], 1, 16), 32, kBigCountSmem, s, R.ia.p,
+      BN_LAUNCH(k_rap_count_big, grid_for(rc.count[1], 1, 6), kCountThreads, kBigCountSmem, s, R.ia.p,
                 R.ja.p, A.ia.p, A.ja.p, P.ia.p, P.ja.p, L1, rc.count[1], cnt.p);
     if (rc.count[2]) {
       const int m = rc.count[2];
@@ -946,7 +983,7 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
       BN_LAUNCH(k_rap_huge_caps, grid_for(m, 128), 128, 0, s, ub.p, L2, m, nc, toff.p);
       long long total = scan_counts64(toff.p, m, s);
       DBuf<int> gkeys((size_t)total, s);
-      BN_LAUNCH(k_rap_count_huge, grid_for((long long)m * 32, 128), 128, 0, s, R.ia.p, R.ja.p,
+      BN_LAUNCH(k_rap_count_huge, grid_for(m, 1, 8), kCountThreads, 0, s, R.ia.p, R.ja.p,
                 A.ia.p, A.ja.p, P.ia.p, P.ja.p, L2, m, toff.p, gkeys.p, cnt.p);
     }
   }
