@@ -37,13 +37,42 @@ template <> __device__ __forceinline__ float bsub(float a, float b) { return __f
 enum { BM_Y = 0, BM_RES = 1, BM_ADD = 2 };
 constexpr int kLongWarps = 32;  // warps per block for rows longer than kLongRow
 
+// A lane's two columns: with K = 64 (PAIR) the neighbours 2 lane and 2 lane + 1,
+// moved as one 8- or 16-byte access, else lane and lane + 32 where they exist.
+template <class T> struct Pair;
+template <> struct Pair<float> { using V = float2; };
+template <> struct Pair<double> { using V = double2; };
+template <class T, bool PAIR>
+__device__ __forceinline__ void row_load(const T* row, int lane, bool c0, bool c1, T& x0, T& x1) {
+  if constexpr (PAIR) {
+    const typename Pair<T>::V v = reinterpret_cast<const typename Pair<T>::V*>(row)[lane];
+    x0 = v.x;
+    x1 = v.y;
+  } else {
+    x0 = c0 ? row[lane] : T(0);
+    x1 = c1 ? row[lane + 32] : T(0);
+  }
+}
+template <class T, bool PAIR>
+__device__ __forceinline__ void row_store(T* row, int lane, bool c0, bool c1, T x0, T x1) {
+  if constexpr (PAIR) {
+    typename Pair<T>::V v;
+    v.x = x0;
+    v.y = x1;
+    reinterpret_cast<typename Pair<T>::V*>(row)[lane] = v;
+  } else {
+    if (c0) row[lane] = x0;
+    if (c1) row[lane + 32] = x1;
+  }
+}
+
 // Row sum of a warp over entries k0..k1-1 in storage order: the lanes load
 // 32 entries at a time (one coalesced read of ja and a), then every entry is
 // broadcast by shuffle and each lane accumulates its columns, so the x
 // gathers of consecutive entries do not wait on one another's index loads.
 // SUB: s -= a_ij x_j (triangular rows) instead of s += ; DIAG >= 0: the
 // entry with column DIAG is not summed, its value goes to *d.
-template <class T, bool SUB>
+template <class T, bool SUB, bool PAIR = false>
 __device__ __forceinline__ void warp_row_sum(int k0, int k1, const int* __restrict__ ja,
                                              const T* __restrict__ a, const T* X, int K,
                                              int lane, bool c0, bool c1, int diag, T& s0, T& s1,
@@ -57,6 +86,43 @@ __device__ __forceinline__ void warp_row_sum(int k0, int k1, const int* __restri
       av = a[kk];
     }
     const int m = min(32, k1 - base);
+    if constexpr (PAIR) {
+      int e = 0;
+      for (; e + 8 <= m; e += 8) {  // eight gathers in flight
+        T x0[8], x1[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+          row_load<T, true>(X + (size_t)__shfl_sync(0xffffffffu, jv, e + u) * K, lane, c0, c1,
+                            x0[u], x1[u]);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const int j = __shfl_sync(0xffffffffu, jv, e + u);
+          const T v = __shfl_sync(0xffffffffu, av, e + u);
+          if (j == diag) {
+            *d = v;
+            if (hit) *hit = true;
+          } else {
+            s0 = badd(s0, bmul(v, x0[u]));
+            s1 = badd(s1, bmul(v, x1[u]));
+          }
+        }
+      }
+#pragma unroll 4
+      for (; e < m; e++) {
+        const int j = __shfl_sync(0xffffffffu, jv, e);
+        const T v = __shfl_sync(0xffffffffu, av, e);
+        if (j == diag) {
+          *d = v;
+          if (hit) *hit = true;
+          continue;
+        }
+        T x0, x1;
+        row_load<T, true>(X + (size_t)j * K, lane, c0, c1, x0, x1);
+        s0 = badd(s0, bmul(v, x0));
+        s1 = badd(s1, bmul(v, x1));
+      }
+      continue;
+    }
 #pragma unroll 4
     for (int e = 0; e < m; e++) {
       const int j = __shfl_sync(0xffffffffu, jv, e);
@@ -78,28 +144,104 @@ __device__ __forceinline__ void warp_row_sum(int k0, int k1, const int* __restri
   }
 }
 
+// Rows r0 .. r0 + n - 1 of a matrix, a warp each, fin(t, s0, s1, d) with the
+// row's sums (t: row minus r0).  A warp adds a row's entries one after the other,
+// so on coarse levels the launch waited for its longest rows (400k network, 64
+// columns: 840 colour-class launches of 75 us each, most of it rows of 128 to
+// 1024 entries).  SPLIT (levels with rows over kSplitRow entries): the block's
+// eight warps take such a row together, consecutive pieces combined in order
+// (line at 64 or 128 entries: the same, at 256: 7 % slower solves).  The barrier
+// this needs per eight rows is left out where every row is short (fine levels).
+// PAIR (split levels at 64 columns): eight gathers of both columns in flight
+// (split colour classes 74 -> 50 us a launch; on rows of five entries the
+// plain form is faster, 123 against 162 us for the finest residual).
+constexpr int kSplitRow = 128;
+template <class T, bool SPLIT, bool PAIR, class F>
+__device__ __forceinline__ void block_rows(const int* __restrict__ ia, const int* __restrict__ ja,
+                                           const T* __restrict__ a, int r0, int n, int skip_long,
+                                           bool gs, const T* X, int K, F fin) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool c0 = lane < K, c1 = lane + 32 < K;
+  if constexpr (!SPLIT) {
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n; t += nw) {
+      const int i = r0 + t, k0 = ia[i], k1 = ia[i + 1];
+      if (skip_long && k1 - k0 > kLongRow) continue;
+      T s0 = T(0), s1 = T(0), d = T(1);
+      warp_row_sum<T, false, PAIR>(k0, k1, ja, a, X, K, lane, c0, c1, gs ? i : -1, s0, s1, &d);
+      fin(t, s0, s1, d);
+    }
+  } else {
+    __shared__ T part[kBlkWarps][kMaxK];
+    __shared__ int split[kBlkWarps];  // the block's rows to split (-1: none of this warp)
+    __shared__ T diag;
+    for (int base = blockIdx.x * kBlkWarps; base < n; base += gridDim.x * kBlkWarps) {
+      const int t = base + w;
+      int len = 0, k0 = 0;
+      if (t < n) {
+        k0 = ia[r0 + t];
+        len = ia[r0 + t + 1] - k0;
+        if (skip_long && len > kLongRow) len = -1;
+      }
+      const bool mine = t < n && len >= 0, big = len > kSplitRow;
+      if (lane == 0) split[w] = big ? t : -1;
+      if (mine && !big) {
+        T s0 = T(0), s1 = T(0), d = T(1);
+        warp_row_sum<T, false, PAIR>(k0, k0 + len, ja, a, X, K, lane, c0, c1, gs ? r0 + t : -1, s0, s1,
+                               &d);
+        fin(t, s0, s1, d);
+      }
+      __syncwarp();
+      if (!__syncthreads_or(big)) continue;
+      for (int q = 0; q < kBlkWarps; q++) {
+        const int tq = split[q];
+        if (tq < 0) continue;  // uniform
+        const int i = r0 + tq, q0 = ia[i], q1 = ia[i + 1];
+        const int per = (q1 - q0 + kBlkWarps - 1) / kBlkWarps;
+        const int p0 = min(q1, q0 + w * per), p1 = min(q1, p0 + per);
+        T s0 = T(0), s1 = T(0), d = T(1);
+        bool hit = false;
+        if (threadIdx.x == 0) diag = T(1);
+        __syncthreads();
+        warp_row_sum<T, false, PAIR>(p0, p1, ja, a, X, K, lane, c0, c1, gs ? i : -1, s0, s1, &d, &hit);
+        if (hit && lane == 0) diag = d;
+        part[w][lane] = s0;
+        part[w][lane + 32] = s1;
+        __syncthreads();
+        if (w == q) {
+          T t0 = T(0), t1 = T(0);
+          for (int u = 0; u < kBlkWarps; u++) {
+            t0 = badd(t0, part[u][lane]);
+            t1 = badd(t1, part[u][lane + 32]);
+          }
+          fin(tq, t0, t1, diag);
+        }
+        __syncthreads();
+      }
+      __syncthreads();  // every warp has read split before the next round writes it
+    }
+  }
+}
+
 // ---------------------------------------------------------------- SpMM
 // Y = A X | B - A X | Y + A X for the rows of [0, n) (rows longer than
 // kLongRow skipped when skip_long: k_spmm_long takes them)
-template <class T, int MODE>
+template <class T, int MODE, bool SPLIT, bool PAIR>
 __global__ void __launch_bounds__(32 * kBlkWarps)
 k_spmm(const int* __restrict__ ia, const int* __restrict__ ja, const T* __restrict__ a, int n,
        const T* __restrict__ X, const T* __restrict__ B, T* __restrict__ Y, int K, int skip_long) {
   const int lane = threadIdx.x & 31;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
   const bool c0 = lane < K, c1 = lane + 32 < K;
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
-    const int k0 = ia[i], k1 = ia[i + 1];
-    if (skip_long && k1 - k0 > kLongRow) continue;
-    T s0 = T(0), s1 = T(0);
-    warp_row_sum<T, false>(k0, k1, ja, a, X, K, lane, c0, c1, -1, s0, s1, nullptr);
+  block_rows<T, SPLIT, PAIR>(ia, ja, a, 0, n, skip_long, false, X, K, [&](int i, T s0, T s1, T) {
     T* yr = Y + (size_t)i * K;
-    const T* br = B ? B + (size_t)i * K : nullptr;
-    if (c0) yr[lane] = MODE == BM_Y ? s0 : (MODE == BM_RES ? bsub(br[lane], s0) : badd(yr[lane], s0));
-    if (c1)
-      yr[lane + 32] =
-          MODE == BM_Y ? s1 : (MODE == BM_RES ? bsub(br[lane + 32], s1) : badd(yr[lane + 32], s1));
-  }
+    if (MODE != BM_Y) {
+      T b0, b1;
+      row_load<T, PAIR>(MODE == BM_RES ? B + (size_t)i * K : yr, lane, c0, c1, b0, b1);
+      s0 = MODE == BM_RES ? bsub(b0, s0) : badd(b0, s0);
+      s1 = MODE == BM_RES ? bsub(b1, s1) : badd(b1, s1);
+    }
+    row_store<T, PAIR>(yr, lane, c0, c1, s0, s1);
+  });
 }
 
 // a block of kLongWarps warps per long row: warp w sums the w-th of
@@ -145,34 +287,25 @@ k_spmm_long(const int* __restrict__ ia, const int* __restrict__ ja, const T* __r
   }
 }
 
-template <class T>
-void spmm(int mode, const DevMat<T>& A, const T* X, const T* B, T* Y, int K, cudaStream_t s) {
-  if (A.n == 0) return;
+template <class T, int MODE>
+void spmm_mode(const DevMat<T>& A, const T* X, const T* B, T* Y, int K, cudaStream_t s) {
   const int g = grid_for((long long)A.n * 32, 32 * kBlkWarps, 8);
   const int skip = A.lrows != nullptr && A.nlong > 0;
   const int gl = A.nlong < 4096 ? A.nlong : 4096;
-  switch (mode) {
-    case BM_Y:
-      BN_LAUNCH((k_spmm<T, BM_Y>), g, 32 * kBlkWarps, 0, s, A.ia, A.ja, A.val, A.n, X, B, Y, K, skip);
-      if (skip)
-        BN_LAUNCH((k_spmm_long<T, BM_Y>), gl, 32 * kLongWarps, 0, s, A.ia, A.ja, A.val, A.lrows,
-                  A.nlong, X, B, Y, K);
-      break;
-    case BM_RES:
-      BN_LAUNCH((k_spmm<T, BM_RES>), g, 32 * kBlkWarps, 0, s, A.ia, A.ja, A.val, A.n, X, B, Y, K,
-                skip);
-      if (skip)
-        BN_LAUNCH((k_spmm_long<T, BM_RES>), gl, 32 * kLongWarps, 0, s, A.ia, A.ja, A.val, A.lrows,
-                  A.nlong, X, B, Y, K);
-      break;
-    default:
-      BN_LAUNCH((k_spmm<T, BM_ADD>), g, 32 * kBlkWarps, 0, s, A.ia, A.ja, A.val, A.n, X, B, Y, K,
-                skip);
-      if (skip)
-        BN_LAUNCH((k_spmm_long<T, BM_ADD>), gl, 32 * kLongWarps, 0, s, A.ia, A.ja, A.val, A.lrows,
-                  A.nlong, X, B, Y, K);
-      break;
-  }
+  const bool split = A.maxrow > kSplitRow, pair = K == kMaxK;
+  auto k = !split ? k_spmm<T, MODE, false, false>
+                  : pair ? k_spmm<T, MODE, true, true> : k_spmm<T, MODE, true, false>;
+  BN_LAUNCH(k, g, 32 * kBlkWarps, 0, s, A.ia, A.ja, A.val, A.n, X, B, Y, K, skip);
+  if (skip)
+    BN_LAUNCH((k_spmm_long<T, MODE>), gl, 32 * kLongWarps, 0, s, A.ia, A.ja, A.val, A.lrows,
+              A.nlong, X, B, Y, K);
+}
+template <class T>
+void spmm(int mode, const DevMat<T>& A, const T* X, const T* B, T* Y, int K, cudaStream_t s) {
+  if (A.n == 0) return;
+  if (mode == BM_Y) spmm_mode<T, BM_Y>(A, X, B, Y, K, s);
+  else if (mode == BM_RES) spmm_mode<T, BM_RES>(A, X, B, Y, K, s);
+  else spmm_mode<T, BM_ADD>(A, X, B, Y, K, s);
 }
 
 // ---------------------------------------------------------------- smoothers
@@ -180,22 +313,19 @@ void spmm(int mode, const DevMat<T>& A, const T* X, const T* B, T* Y, int K, cud
 // numbering, the last nlong of them long): x_i = (b_i - sum_{j != i} a_ij
 // x_j) / a_ii (1 without a diagonal entry), written to X in place or, for an
 // overflow (Jacobi) class, to OUT row t.
-template <class T>
+template <class T, bool SPLIT, bool PAIR>
 __global__ void __launch_bounds__(32 * kBlkWarps)
 k_gsm(const int* __restrict__ ia, const int* __restrict__ ja, const T* __restrict__ a, int r0,
       int nshort, const T* __restrict__ B, T* X, T* __restrict__ OUT, int K) {
   const int lane = threadIdx.x & 31;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
   const bool c0 = lane < K, c1 = lane + 32 < K;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nshort; t += nw) {
+  block_rows<T, SPLIT, PAIR>(ia, ja, a, r0, nshort, 0, true, X, K, [&](int t, T s0, T s1, T d) {
     const int i = r0 + t;
-    T s0 = T(0), s1 = T(0), d = T(1);
-    warp_row_sum<T, false>(ia[i], ia[i + 1], ja, a, X, K, lane, c0, c1, i, s0, s1, &d);
-    const T* br = B + (size_t)i * K;
-    T* o = OUT ? OUT + (size_t)t * K : X + (size_t)i * K;
-    if (c0) o[lane] = bsub(br[lane], s0) / d;
-    if (c1) o[lane + 32] = bsub(br[lane + 32], s1) / d;
-  }
+    T b0, b1;
+    row_load<T, PAIR>(B + (size_t)i * K, lane, c0, c1, b0, b1);
+    row_store<T, PAIR>(OUT ? OUT + (size_t)t * K : X + (size_t)i * K, lane, c0, c1,
+                       bsub(b0, s0) / d, bsub(b1, s1) / d);
+  });
 }
 
 template <class T>
@@ -240,9 +370,11 @@ template <class T>
 void gs_class_block(const DevMat<T>& A, int r0, int nr, int nlong, const T* B, T* X, T* OUT,
                     int K, cudaStream_t s) {
   const int nshort = nr - nlong;
+  const int g = grid_for((long long)nshort * 32, 32 * kBlkWarps, 8);
+  const bool split = A.maxrow > kSplitRow, pair = K == kMaxK;
+  auto k = !split ? k_gsm<T, false, false> : pair ? k_gsm<T, true, true> : k_gsm<T, true, false>;
   if (nshort > 0)
-    BN_LAUNCH(k_gsm<T>, grid_for((long long)nshort * 32, 32 * kBlkWarps, 8), 32 * kBlkWarps, 0, s,
-              A.ia, A.ja, A.val, r0, nshort, B, X, OUT, K);
+    BN_LAUNCH(k, g, 32 * kBlkWarps, 0, s, A.ia, A.ja, A.val, r0, nshort, B, X, OUT, K);
   if (nlong > 0)
     BN_LAUNCH(k_gsm_long<T>, nlong < 4096 ? nlong : 4096, 32 * kLongWarps, 0, s, A.ia, A.ja, A.val,
               r0, nshort, nlong, B, X, OUT, K);
@@ -604,7 +736,8 @@ __global__ void k_dot_finish(const double* __restrict__ partial, int nb, int K,
   const int c = threadIdx.x;
   if (c >= K) return;
   double t = 0.0;
-  for (int b = 0; b < nb; b++) t += partial[(size_t)b * K + c];
+#pragma unroll 16
+  for (int b = 0; b < nb; b++) t += partial[(size_t)b * K + c];  // loads ahead of the sum
   out[c] = t;
 }
 

@@ -41,6 +41,7 @@ struct DevMat {
   int group = 0;
   const int* lrows = nullptr;
   int nlong = 0;
+  int maxrow = 0;              // entries of the longest row (0: not known)
   const int* tiles = nullptr;  // row-tile kernel: order in which tiles are visited (null: natural)
 };
 

@@ -457,6 +457,7 @@ DevMat<T> Solver::mat(const CSR& M, const DBuf<float>* v32, const RowLayout* lay
     d.group = lay->group;
     d.lrows = lay->lrows.p;
     d.nlong = lay->nlong;
+    d.maxrow = lay->maxrow;
     d.tiles = lay->tiles.n ? lay->tiles.p : nullptr;
   }
   return d;

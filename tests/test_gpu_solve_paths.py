@@ -168,3 +168,42 @@ def test_tail_after_the_hierarchy_changes(monkeypatch):
     for k, (x, y) in enumerate(zip(tail, plain)):
         tol = TOL[amg.PREC_MIXED if k == 4 else amg.PREC_FP64]
         assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y), k
+
+
+@pytest.mark.parametrize("precision", [amg.PREC_FP64, amg.PREC_MIXED])
+@pytest.mark.parametrize("k", [1, 5, 33, 64])
+@pytest.mark.parametrize("deg", [62, 63, 64, 65, 600, 1022, 1023, 1024])
+def test_block_rows_split_over_the_warps(deg, k, precision):
+    """Many right-hand sides over rows at and around the lengths that a block's
+    warps share (64) and that a block of their own takes (1024): every column
+    meets the tolerance on the true residual."""
+    import scipy.sparse as sp
+    n, ia, ja, val = hub_matrix(side=40, hubs=(deg, deg), weak_hubs=(), seed=deg)
+    A = sp.csr_matrix((val, ja, ia), shape=(n, n))
+    B = np.random.default_rng(k).standard_normal((n, k))
+    s = amg.AMGSolver(n, ia, ja, val, min_size=100, precision=precision, stop=amg.STOP_RELRES)
+    X, its, rel, rc = s.solve_block(B, tol=1e-9)
+    single = s.solve(np.ascontiguousarray(B[:, 0]), tol=1e-9)[1]
+    s.close()
+    assert rc == 0 and abs(its[0] - single) <= 1
+    r = np.linalg.norm(B - A @ X, axis=0) / np.linalg.norm(B, axis=0)
+    assert (r <= 1.01e-9).all()
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_block_rows_split_in_some_rounds_only(seed):
+    """More rows than the grid's warps, so that a block takes several rounds of
+    eight rows, some of them with a row to share and most without."""
+    import scipy.sparse as sp
+    n, ia, ja, val = hub_matrix(side=130, hubs=(70, 90, 200, 65, 400, 300) * 20, weak_hubs=(),
+                                seed=seed)
+    q = np.random.default_rng(seed).permutation(n)
+    A = sp.csr_matrix((val, ja, ia), shape=(n, n))[q][:, q].tocsr()
+    A.sort_indices()
+    B = np.random.default_rng(seed).standard_normal((n, 64))
+    s = amg.AMGSolver(n, A.indptr, A.indices, A.data, min_size=300, precision=amg.PREC_MIXED,
+                      stop=amg.STOP_RELRES)
+    X, its, rel, rc = s.solve_block(B, tol=1e-9)
+    s.close()
+    r = np.linalg.norm(B - A @ X, axis=0) / np.linalg.norm(B, axis=0)
+    assert rc == 0 and (r <= 1.01e-9).all()
