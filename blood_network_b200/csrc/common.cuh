@@ -71,14 +71,22 @@ extern std::atomic<unsigned long long> g_launch_count;
 // that launch and block scheduling of the next kernel overlap this kernel's
 // tail.  BN_LAUNCH_PDL launches with programmatic stream serialization; only
 // kernels that begin with BN_PDL_ENTRY() may be launched that way (a test
-// checks the sources).  Off unless BN_PDL=1 (measured slower on the 20M
-// solve); with plain launches the entry is a no-op.
+// checks the sources).  On for the solves of the smaller networks (PdlScope,
+// solver.cu), off for the larger; with plain launches the entry is a no-op.
 __device__ __forceinline__ void pdl_entry() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 #define BN_PDL_ENTRY() ::bn::pdl_entry()
 bool pdl_enabled();
+// Programmatic launches on or off for the calling thread while it lives.
+struct PdlScope {
+  bool before;
+  explicit PdlScope(bool on);
+  ~PdlScope();
+  PdlScope(const PdlScope&) = delete;
+  PdlScope& operator=(const PdlScope&) = delete;
+};
 #define BN_LAUNCH_PDL(kern_, grid_, block_, smem_, strm_, ...)                         \
   do {                                                                                  \
     ::bn::g_launch_count++;                                                             \

@@ -18,13 +18,15 @@ namespace bn {
 
 std::atomic<unsigned long long> g_launch_count{0};
 
-// Off by default: on the 20M network the solve measured slower with it
-// (mixed 103.6 ms against 98.5 ms, FP64 139.2 against 122.9 ms, same run);
-// BN_PDL=1 turns it on.
-bool pdl_enabled() {
-  static const bool on = getenv("BN_PDL") != nullptr && atoi(getenv("BN_PDL")) != 0;
-  return on;
+// BN_PDL=0 / 1 decides for every solve, without it the solve at hand by its size
+static bool pdl_rule(bool on) {
+  const char* e = getenv("BN_PDL");
+  return e ? atoi(e) != 0 : on;
 }
+static thread_local bool t_pdl = pdl_rule(false);
+bool pdl_enabled() { return t_pdl; }
+PdlScope::PdlScope(bool on) : before(t_pdl) { t_pdl = pdl_rule(on); }
+PdlScope::~PdlScope() { t_pdl = before; }
 
 bool trace_on() {
   static int on = -1;

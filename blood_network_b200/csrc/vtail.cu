@@ -348,12 +348,14 @@ void tail_run(const TailOp<T>* ops, int op0, int op1, int top_lev, const T* top_
   cfg.blockDim = dim3(kTailThreads);
   cfg.dynamicSmemBytes = sizeof(TailOp<T>) * (size_t)(op1 - op0);
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = nblk;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
   g_launch_count++;
   BN_CUDA(cudaLaunchKernelEx(&cfg, k_tail<T>, ops + op0, op1 - op0, top_lev, top_b, top_x));
 }

@@ -207,3 +207,20 @@ def test_block_rows_split_in_some_rounds_only(seed):
     s.close()
     r = np.linalg.norm(B - A @ X, axis=0) / np.linalg.norm(B, axis=0)
     assert rc == 0 and (r <= 1.01e-9).all()
+
+
+@pytest.mark.parametrize("precision", [amg.PREC_FP64, amg.PREC_MIXED])
+@pytest.mark.parametrize("n", [40, 3000, 60000])
+def test_programmatic_launches_change_nothing(n, precision, monkeypatch):
+    """The same kernels in the same order: a result that differs was read early."""
+    m, ia, ja, val = _vascular(n, False)
+    b = np.random.default_rng(n).standard_normal(m)
+    out = []
+    for pdl in "01":
+        monkeypatch.setenv("BN_PDL", pdl)
+        s = amg.AMGSolver(m, ia, ja, val, precision=precision, stop=amg.STOP_RELRES)
+        x = s.solve(b, tol=1e-8)[0]
+        out.append((s.precond(b), x))
+        s.close()
+    for x, y in zip(*out):
+        assert np.linalg.norm(x - y) <= TOL[precision] * np.linalg.norm(y)
