@@ -403,7 +403,9 @@ __global__ void k_long_rows(const int* __restrict__ ia, int n, int* __restrict__
 
 void analyze_rows(const CSR& A, RowLayout& out, cudaStream_t s) {
   const double avg = A.n > 0 ? (double)A.nnz / A.n : 0.0;
-  out.group = avg <= 8.0 ? 0 : (avg <= 16.0 ? 4 : (avg <= 48.0 ? 8 : 32));
+  // 16 lanes from 36 entries a row on: the fastest choice on the 20M and 4M
+  // networks' levels of 39 to 48 entries (at most 1.5 % of a solve)
+  out.group = avg <= 8.0 ? 0 : avg <= 16.0 ? 4 : avg <= 36.0 ? 8 : avg <= 64.0 ? 16 : 32;
   // BN_SPMV_GROUP=g pins every operator to one kernel variant (0-3: row
   // tiles of 256/128/64/32 rows, 5: staged 256-row tiles, 4/8/16/32: lanes
   // per row); the autotuner may still change it

@@ -486,6 +486,26 @@ static std::vector<int> host_ia(const CSR& M, cudaStream_t s) {
   return h;
 }
 
+// Lanes per row of the Gauss-Seidel classes.  Where the rows alone fill the chip
+// a lane should have four entries or so to itself (its loads overlap), so about
+// a quarter of the mean row; on small levels a launch is one chain of loads, and
+// a lane per entry shortens it.  What timing every choice on a level found best:
+// 75k rows 4, 16, 32 lanes for its levels of 75k, 31k, 11k rows with 5, 9, 18
+// entries; 4M 1, 2, 4, 16 for 5, 9, 17, 39 entries; 20M mixed 1, 1, 4, 16 for
+// 5, 10, 20, 48.  One lane up to 12 entries, 8 up to 48 and 32 beyond for every
+// size (as it was) -> those choices: one solve at 75k 7.03 -> 6.52 ms, 4M 32.0 ->
+// 31.3, 20M 94.2 -> 91.9.
+constexpr int kGsFewRows = 65536;
+static int gs_lanes(int n, double avg) {
+  if (n <= kGsFewRows) {
+    int g = 1;
+    while (g < 32 && g < avg) g *= 2;
+    return g;
+  }
+  if (avg <= 12.0) return n <= 2 * kGsFewRows ? 4 : 1;
+  return avg <= 22.0 ? 4 : avg <= 36.0 ? 8 : avg <= 64.0 ? 16 : 32;
+}
+
 void Solver::color_level(Level& L, int smoother) {
   const int n = L.A.n;
   const int g = grid_for(n, 256);
@@ -580,15 +600,13 @@ void Solver::color_level(Level& L, int smoother) {
     for (int c = 0; c < nc; c++) jac[c] = L.cjac[c];
     L.d_cptr.alloc(nc + 1, s);
     L.d_cptr.upload(L.cptr.data(), nc + 1);
-    L.d_cjac.alloc(nc > 0 ? nc : 1, s);
-    if (nc) L.d_cjac.upload(jac.data(), nc);
     BN_CUDA(cudaStreamSynchronize(s));
   }
   const double avg = n > 0 ? (double)L.A.nnz / n : 0.0;
-  L.gs_group = avg <= 12.0 ? 1 : (avg <= 48.0 ? 8 : 32);
+  L.gs_group = gs_lanes(n, avg);
   // BN_GS_LANES=g pins the Gauss-Seidel kernel (0 staged row tiles, 1/2/4/8/
   // 16/32 lanes per row); the autotuner may still change it
-  static const int gs_forced = getenv("BN_GS_LANES") ? atoi(getenv("BN_GS_LANES")) : -1;
+  const int gs_forced = getenv("BN_GS_LANES") ? atoi(getenv("BN_GS_LANES")) : -1;
   if (gs_forced == 0 || gs_forced == 1 || gs_forced == 2 || gs_forced == 4 || gs_forced == 8 ||
       gs_forced == 16 || gs_forced == 32)
     L.gs_group = gs_forced;

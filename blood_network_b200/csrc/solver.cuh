@@ -39,7 +39,7 @@ struct Level {
   int colored_for = -1;    // smoother the colouring was built for
   int color_rounds = 0;
   int gs_group = 1;        // lanes per row in the GS kernel
-  DBuf<int> d_cptr, d_cjac;  // class tables on the device (single-block sweeps)
+  DBuf<int> d_cptr;  // class bounds on the device
   DBuf<double> l1, dg;
   DBuf<float> l1_32, dg32;
   // load-balanced kernels: packings of Ap, Pp, Rp (one range each) and of

@@ -224,3 +224,18 @@ def test_programmatic_launches_change_nothing(n, precision, monkeypatch):
         s.close()
     for x, y in zip(*out):
         assert np.linalg.norm(x - y) <= TOL[precision] * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("precision", [amg.PREC_FP64, amg.PREC_MIXED])
+@pytest.mark.parametrize("n, per_row", [(65536, 8), (65537, 8), (65537, 16), (65537, 30),
+                                        (65537, 50), (65537, 80), (131073, 8), (3000, 5),
+                                        (3000, 12), (3000, 40)])
+def test_lanes_per_row(n, per_row, precision, monkeypatch):
+    """Both sides of every bound of the rule for the Gauss-Seidel lanes, against
+    one lane per row."""
+    m, ia, ja, val = _random_spd(n, per_row, per_row)
+    g = np.random.default_rng(n).standard_normal(m)
+    x = precond(m, ia, ja, val, g, precision=precision)
+    monkeypatch.setenv("BN_GS_LANES", "1")
+    y = precond(m, ia, ja, val, g, precision=precision)
+    assert np.linalg.norm(x - y) <= TOL[precision] * np.linalg.norm(y)
