@@ -12,9 +12,9 @@
 // the row into a shared-memory open-addressing table in parallel
 // (atomicCAS) and counts the new keys.  Pass 2 keeps the reference's
 // sequential order without serialising the memory traffic: the 32 lanes walk
-// A row i1 together (coalesced), form r*a, expand their P rows into an
-// ordered product stream in shared memory (warp prefix sum), and consume the
-// stream 32 products at a time: lanes holding the same column group up
+// the list of A entries of R's row together (coalesced), expand their P rows
+// into an ordered product stream (warp prefix sums), and consume the stream 32
+// products at a time: lanes holding the same column group up
 // (match_any) and the group's first lane adds the group's products, in
 // stream order, to that column's sum (a new column takes its first product
 // and the next slot in order of first appearance), so every sum is formed in
@@ -32,7 +32,6 @@ namespace bn {
 constexpr int kWarpCap = 1024;    // per-warp table (distinct columns <= 512)
 constexpr int kBigCap = 8192;     // one-warp-per-block table (<= 4096)
 constexpr int kRapWarps = 4;
-constexpr int kBuf = 256;         // product stream chunk
 
 __device__ __forceinline__ unsigned rap_hash(int key, unsigned mask) {
   return ((unsigned)key * 2654435761u >> 7) & mask;
@@ -109,6 +108,114 @@ __global__ void k_rap_bound(const int* __restrict__ ria, const int* __restrict__
   }
 }
 
+// lane of the entry e, given where each lane's entries start (ascending; a lane
+// without entries starts where the next one does)
+__device__ __forceinline__ int entry_lane(int start, int e) {
+  int l = 0;
+#pragma unroll
+  for (int st = 16; st > 0; st >>= 1)
+    if (__shfl_sync(0xffffffffu, start, l + st) <= e) l += st;
+  return l;
+}
+
+__device__ __forceinline__ int warp_total(int v, int lane, int* start) {
+  int incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += u;
+  }
+  *start = incl - v;
+  return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+// A coarse row's products (r*a)*p in the reference's order, up to 32 at a time:
+// use(active, column, r*a, p).  The row is a chain of dependent loads (R's entry,
+// A's row bounds, A's entry, P's row bounds, P's entry), and a launch waits for its
+// longest row.  So R's entries are taken 32 at a time and their A entries as one
+// list of which each lane holds one, whatever rows they are from, and so for the P
+// entries; A's entries are loaded two chunks ahead, P's row bounds one, P's entries
+// one step.  One A row at a time left most lanes idle and waited for the whole
+// chain at each of R's entries (150k-row network, us a level: filling rows of 65 to
+// 512 columns 412 -> 333, of up to 64 columns 130 -> 102; counting rows of 65 to
+// 512 products 224 -> 76).
+template <bool VAL, class F>
+__device__ __forceinline__ void rap_products(int ic, int lane, const int* __restrict__ ria,
+                                             const int* __restrict__ rja,
+                                             const double* __restrict__ rval,
+                                             const int* __restrict__ aia,
+                                             const int* __restrict__ aja,
+                                             const double* __restrict__ aval,
+                                             const int* __restrict__ pia,
+                                             const int* __restrict__ pja,
+                                             const double* __restrict__ pval, F&& use) {
+  const int r1 = ria[ic + 1];
+  for (int kb = ria[ic]; kb < r1; kb += 32) {
+    int a0 = 0, alen = 0, astart;
+    double r = 0.0;
+    if (kb + lane < r1) {
+      const int i1 = rja[kb + lane];
+      if (VAL) r = rval[kb + lane];
+      a0 = aia[i1];
+      alen = aia[i1 + 1] - a0;
+    }
+    const int atotal = warp_total(alen, lane, &astart);
+    int e_i2 = 0;
+    double e_r = 0.0, e_a = 0.0;
+    auto load_a = [&](int eb) {
+      const int l = entry_lane(astart, eb + lane);
+      const int k2 = __shfl_sync(0xffffffffu, a0 - astart, l) + eb + lane;
+      if (VAL) e_r = __shfl_sync(0xffffffffu, r, l);
+      e_i2 = -1;
+      if (eb + lane < atotal) {
+        e_i2 = aja[k2];
+        if (VAL) e_a = aval[k2];
+      }
+    };
+    int p0 = 0, p1 = 0;
+    double ra = 0.0;
+    auto load_pia = [&]() {
+      p0 = p1 = 0;
+      if (e_i2 >= 0) {
+        p0 = pia[e_i2];
+        p1 = pia[e_i2 + 1];
+      }
+      if (VAL) ra = xmul(e_r, e_a);
+    };
+    load_a(0);
+    load_pia();
+    if (32 < atotal) load_a(32);
+    for (int eb = 0; eb < atotal; eb += 32) {
+      int pstart;
+      const int ptotal = warp_total(p1 - p0, lane, &pstart);
+      const int pofs = p0 - pstart;
+      const double ra_now = ra;
+      if (eb + 32 < atotal) {
+        load_pia();
+        if (eb + 64 < atotal) load_a(eb + 64);
+      }
+      int col = 0;
+      double rav = 0.0, pv = 0.0;
+      auto load_p = [&](int q0) {
+        const int l = entry_lane(pstart, q0 + lane);
+        const int k3 = __shfl_sync(0xffffffffu, pofs, l) + q0 + lane;
+        if (VAL) rav = __shfl_sync(0xffffffffu, ra_now, l);
+        if (q0 + lane < ptotal) {
+          col = pja[k3];
+          if (VAL) pv = pval[k3];
+        }
+      };
+      if (ptotal > 0) load_p(0);
+      for (int q0 = 0; q0 < ptotal; q0 += 32) {
+        const int c = col;
+        const double x = rav, y = pv;
+        if (q0 + 32 < ptotal) load_p(q0 + 32);
+        use(q0 + lane < ptotal, c, x, y);
+      }
+    }
+  }
+}
+
 __device__ int rap_count_row(int ic, Table t, int lane, const int* __restrict__ ria,
                              const int* __restrict__ rja, const int* __restrict__ aia,
                              const int* __restrict__ aja, const int* __restrict__ pia,
@@ -117,13 +224,10 @@ __device__ int rap_count_row(int ic, Table t, int lane, const int* __restrict__ 
   __syncwarp();
   int cnt = 0;
   if (lane == 0) cnt += table_insert_atomic(t, ic);
-  for (int k1 = ria[ic]; k1 < ria[ic + 1]; k1++) {
-    const int i1 = rja[k1];
-    for (int k2 = aia[i1] + lane; k2 < aia[i1 + 1]; k2 += 32) {
-      const int i2 = aja[k2];
-      for (int k3 = pia[i2]; k3 < pia[i2 + 1]; k3++) cnt += table_insert_atomic(t, pja[k3]);
-    }
-  }
+  rap_products<false>(ic, lane, ria, rja, nullptr, aia, aja, nullptr, pia, pja, nullptr,
+                      [&](bool act, int col, double, double) {
+                        if (act) cnt += table_insert_atomic(t, col);
+                      });
   for (int off = 16; off > 0; off >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
   __syncwarp();
   return cnt;
@@ -151,8 +255,8 @@ __device__ __forceinline__ void table_put(Table t, int key, int slot) {
   }
 }
 
-template <int BUF = kBuf>
-__device__ void rap_fill_row(int ic, Table t, int lane, int* bcol, double* bval,
+// bval: 32 products of the warp
+__device__ void rap_fill_row(int ic, Table t, int lane, double* bval,
                              const int* __restrict__ ria, const int* __restrict__ rja,
                              const double* __restrict__ rval, const int* __restrict__ aia,
                              const int* __restrict__ aja, const double* __restrict__ aval,
@@ -169,82 +273,45 @@ __device__ void rap_fill_row(int ic, Table t, int lane, int* bcol, double* bval,
   __syncwarp();
   int nslots = 1;  // warp-uniform
   const unsigned lt = (1u << lane) - 1u;
-  for (int k1 = ria[ic]; k1 < ria[ic + 1]; k1++) {
-    const double r = rval[k1];
-    const int i1 = rja[k1];
-    const int a1 = aia[i1 + 1];
-    for (int base = aia[i1]; base < a1; base += 32) {
-      const int k2 = base + lane;
-      double ra = 0.0;
-      int p0 = 0, plen = 0;
-      if (k2 < a1) {
-        ra = xmul(r, aval[k2]);
-        const int i2 = aja[k2];
-        p0 = pia[i2];
-        plen = pia[i2 + 1] - p0;
-      }
-      // exclusive prefix of plen across the warp (stream positions)
-      int incl = plen;
-      for (int off = 1; off < 32; off <<= 1) {
-        int v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += v;
-      }
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      const int start = incl - plen;
-      (void)lt;
-      for (int cs = 0; cs < total; cs += BUF) {
-        for (int q = 0; q < plen; q++) {
-          const int sidx = start + q - cs;
-          if (sidx >= 0 && sidx < BUF) {
-            bcol[sidx] = pja[p0 + q];
-            bval[sidx] = xmul(ra, pval[p0 + q]);
-          }
-        }
+  // the stream in order, 32 products at a time: lanes holding the same column
+  // form a group whose lowest lane adds the group's products to that column's
+  // sum in stream order (a new column takes its first product and the next
+  // slot, numbered in order of first appearance); distinct columns proceed in
+  // parallel
+  rap_products<true>(
+      ic, lane, ria, rja, rval, aia, aja, aval, pia, pja, pval,
+      [&](bool act, int c, double ra, double p) {
+        const double v = xmul(ra, p);
+        bval[lane] = v;
+        const int col = act ? c : -1 - lane;
+        const unsigned grp = __match_any_sync(0xffffffffu, col);
+        const bool lead = act && (__ffs(grp) - 1 == lane);
+        int slot = lead ? table_find_slot(t, col) : 0;
+        const unsigned newm = __ballot_sync(0xffffffffu, lead && slot < 0);
         __syncwarp();
-        // consume the stream in order, 32 products at a time: lanes holding
-        // the same column form a group whose lowest lane adds the group's
-        // products to that column's sum in stream order (a new column takes
-        // its first product and the next slot, numbered in order of first
-        // appearance); distinct columns proceed in parallel
-        const int m = min(BUF, total - cs);
-        for (int q0 = 0; q0 < m; q0 += 32) {
-          const int q = q0 + lane;
-          const bool act = q < m;
-          const int col = act ? bcol[q] : -1 - lane;
-          const unsigned grp = __match_any_sync(0xffffffffu, col);
-          const bool lead = act && (__ffs(grp) - 1 == lane);
-          int slot = lead ? table_find_slot(t, col) : 0;
-          const unsigned newm = __ballot_sync(0xffffffffu, lead && slot < 0);
-          if (lead) {
-            double acc;
-            unsigned g = grp;
-            if (slot < 0) {
-              slot = nslots + __popc(newm & lt);
-              table_put(t, col, slot);
-              cja[cbase + slot] = col;
-              acc = bval[q];
-              g &= g - 1;
-            } else {
-              acc = t.vals[slot];
-            }
-            for (; g; g &= g - 1) acc = xadd(acc, bval[q0 + __ffs(g) - 1]);
-            t.vals[slot] = acc;
+        if (lead) {
+          double acc;
+          if (slot < 0) {
+            slot = nslots + __popc(newm & lt);
+            table_put(t, col, slot);
+            cja[cbase + slot] = col;
+            acc = v;
+          } else {
+            acc = xadd(t.vals[slot], v);
           }
-          nslots += __popc(newm);
-          __syncwarp();
+          for (unsigned g = grp & (grp - 1); g; g &= g - 1) acc = xadd(acc, bval[__ffs(g) - 1]);
+          t.vals[slot] = acc;
         }
-      }
-    }
-  }
+        nslots += __popc(newm);
+        __syncwarp();
+      });
   for (int q = lane; q < nslots; q += 32) cval[cbase + q] = t.vals[q];
   __syncwarp();
 }
 
-// ---------------- small rows (at most kSmallCap/2 products): small tables
-// and stream buffers, so that many more warps per SM hide the latency of the
+// ---------------- small rows (at most kSmallCap/2 products): small tables, so that many more warps per SM hide the latency of the
 // R -> A -> P walk (the fine and first coarse levels are almost all small)
 constexpr int kSmallCap = 128;
-constexpr int kSmallBuf = 64;
 constexpr int kSmallWarps = 8;
 
 __global__ void __launch_bounds__(32 * kSmallWarps)
@@ -270,16 +337,15 @@ k_rap_fill_small(const int* __restrict__ ria, const int* __restrict__ rja,
                  const double* __restrict__ pval, const int* __restrict__ rows, int m,
                  const int* __restrict__ cia, int* __restrict__ cja, double* __restrict__ cval) {
   __shared__ double vals_s[kSmallWarps][kSmallCap / 2];
-  __shared__ double bval_s[kSmallWarps][kSmallBuf];
+  __shared__ double bval_s[kSmallWarps][32];
   __shared__ int keys_s[kSmallWarps][kSmallCap];
   __shared__ int slots_s[kSmallWarps][kSmallCap];
-  __shared__ int bcol_s[kSmallWarps][kSmallBuf];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   Table t{keys_s[w], slots_s[w], vals_s[w], kSmallCap - 1};
   for (int q = blockIdx.x * kSmallWarps + w; q < m; q += gridDim.x * kSmallWarps) {
     const int ic = rows[q];
-    rap_fill_row<kSmallBuf>(ic, t, lane, bcol_s[w], bval_s[w], ria, rja, rval, aia, aja, aval,
-                            pia, pja, pval, cia[ic], cja, cval);
+    rap_fill_row(ic, t, lane, bval_s[w], ria, rja, rval, aia, aja, aval, pia, pja, pval, cia[ic],
+                 cja, cval);
   }
 }
 
@@ -372,21 +438,17 @@ k_rap_count_huge(const int* __restrict__ ria, const int* __restrict__ rja,
 
 // ---------------- pass 2 kernels
 constexpr size_t kWarpFillSmem =
-    kRapWarps * (kWarpCap * 2 * sizeof(int) + (kWarpCap / 2) * sizeof(double) +
-                 kBuf * (sizeof(int) + sizeof(double)));
+    kRapWarps * (kWarpCap * 2 * sizeof(int) + (kWarpCap / 2 + 32) * sizeof(double));
 constexpr size_t kBigFillSmem =
-    kBigCap * 2 * sizeof(int) + (kBigCap / 2) * sizeof(double) + kBuf * (sizeof(int) + sizeof(double));
+    kBigCap * 2 * sizeof(int) + (kBigCap / 2 + 32) * sizeof(double);
 constexpr size_t kBigCountSmem = kBigCap * sizeof(int);
 
-__device__ __forceinline__ void carve(unsigned char* base, int cap, Table* t, int** bcol,
-                                      double** bval) {
+__device__ __forceinline__ void carve(unsigned char* base, int cap, Table* t, double** bval) {
   double* vals = (double*)base;                       // cap/2 doubles
-  double* bv = vals + cap / 2;                        // kBuf doubles
-  int* keys = (int*)(bv + kBuf);                      // cap ints
+  double* bv = vals + cap / 2;                        // 32 doubles
+  int* keys = (int*)(bv + 32);                        // cap ints
   int* slots = keys + cap;                            // cap ints
-  int* bc = slots + cap;                              // kBuf ints
   *t = Table{keys, slots, vals, (unsigned)cap - 1};
-  *bcol = bc;
   *bval = bv;
 }
 
@@ -400,12 +462,11 @@ k_rap_fill_warp(const int* __restrict__ ria, const int* __restrict__ rja,
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   Table t;
-  int* bcol;
   double* bval;
-  carve(smem + w * (kWarpFillSmem / kRapWarps), kWarpCap, &t, &bcol, &bval);
+  carve(smem + w * (kWarpFillSmem / kRapWarps), kWarpCap, &t, &bval);
   for (int q = blockIdx.x * kRapWarps + w; q < m; q += gridDim.x * kRapWarps) {
     const int ic = rows[q];
-    rap_fill_row(ic, t, lane, bcol, bval, ria, rja, rval, aia, aja, aval, pia, pja, pval, cia[ic],
+    rap_fill_row(ic, t, lane, bval, ria, rja, rval, aia, aja, aval, pia, pja, pval, cia[ic],
                  cja, cval);
   }
 }
@@ -420,37 +481,36 @@ k_rap_fill_big(const int* __restrict__ ria, const int* __restrict__ rja,
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   Table t;
-  int* bcol;
   double* bval;
-  carve(smem, kBigCap, &t, &bcol, &bval);
+  carve(smem, kBigCap, &t, &bval);
   for (int q = blockIdx.x; q < m; q += gridDim.x) {
     const int ic = rows[q];
-    rap_fill_row(ic, t, lane, bcol, bval, ria, rja, rval, aia, aja, aval, pia, pja, pval, cia[ic],
+    rap_fill_row(ic, t, lane, bval, ria, rja, rval, aia, aja, aval, pia, pja, pval, cia[ic],
                  cja, cval);
   }
 }
 
-__global__ void k_rap_fill_huge(const int* __restrict__ ria, const int* __restrict__ rja,
+__global__ void __launch_bounds__(32 * kRapWarps)
+k_rap_fill_huge(const int* __restrict__ ria, const int* __restrict__ rja,
                                 const double* __restrict__ rval, const int* __restrict__ aia,
                                 const int* __restrict__ aja, const double* __restrict__ aval,
                                 const int* __restrict__ pia, const int* __restrict__ pja,
                                 const double* __restrict__ pval, const int* __restrict__ rows,
                                 int m, const long long* __restrict__ toff,
                                 int* __restrict__ gkeys, int* __restrict__ gslots,
-                                double* __restrict__ gvals, int* __restrict__ gbcol,
-                                double* __restrict__ gbval, const int* __restrict__ cia,
+                                double* __restrict__ gvals, const int* __restrict__ cia,
                                 int* __restrict__ cja, double* __restrict__ cval) {
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  int* bcol = gbcol + (size_t)wid * kBuf;
-  double* bval = gbval + (size_t)wid * kBuf;
+  __shared__ double bval_s[kRapWarps][32];
+  double* bval = bval_s[threadIdx.x >> 5];
   for (int q = wid; q < m; q += warps) {
     const int ic = rows[q];
     const long long off = toff[q];
     const unsigned cap = (unsigned)(toff[q + 1] - off);
     Table t{gkeys + off, gslots + off, gvals + off / 2, cap - 1};
-    rap_fill_row(ic, t, lane, bcol, bval, ria, rja, rval, aia, aja, aval, pia, pja, pval, cia[ic],
+    rap_fill_row(ic, t, lane, bval, ria, rja, rval, aia, aja, aval, pia, pja, pval, cia[ic],
                  cja, cval);
   }
 }
@@ -1039,13 +1099,11 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
       toff.zero();
       BN_LAUNCH(k_rap_huge_caps, grid_for(m, 128), 128, 0, s, exact.p, L2, m, nc, toff.p);
       long long total = scan_counts64(toff.p, m, s);
-      const int grid = grid_for((long long)m * 32, 128);
-      const size_t nwarps = (size_t)grid * 4;
-      DBuf<int> gkeys((size_t)total, s), gslots((size_t)total, s), gbcol(nwarps * kBuf, s);
-      DBuf<double> gvals((size_t)total / 2 + 1, s), gbval(nwarps * kBuf, s);
-      BN_LAUNCH(k_rap_fill_huge, grid, 128, 0, s, R.ia.p, R.ja.p, R.val.p, A.ia.p, A.ja.p,
+      DBuf<int> gkeys((size_t)total, s), gslots((size_t)total, s);
+      DBuf<double> gvals((size_t)total / 2 + 1, s);
+      BN_LAUNCH(k_rap_fill_huge, grid_for(m, kRapWarps), 32 * kRapWarps, 0, s, R.ia.p, R.ja.p, R.val.p, A.ia.p, A.ja.p,
                 A.val.p, P.ia.p, P.ja.p, P.val.p, L2, m, toff.p, gkeys.p, gslots.p, gvals.p,
-                gbcol.p, gbval.p, Ac.ia.p, Ac.ja.p, Ac.val.p);
+                Ac.ia.p, Ac.ja.p, Ac.val.p);
     }
   }
 }
