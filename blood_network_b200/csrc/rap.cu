@@ -20,9 +20,8 @@
 // and the next slot in order of first appearance), so every sum is formed in
 // exactly the reference's order while distinct columns proceed in parallel.
 // Rows with at most 64 products use small per-warp tables (many resident
-// warps); rows whose column count exceeds the per-warp table use a one-warp
-// block with a large dynamic table, and beyond that a table in global
-// memory.
+// warps); rows with many products or more columns than the per-warp table
+// holds use a block, and beyond its table one in global memory.
 #include "internal.cuh"
 
 #include <cub/cub.cuh>
@@ -30,8 +29,9 @@
 namespace bn {
 
 constexpr int kWarpCap = 1024;    // per-warp table (distinct columns <= 512)
-constexpr int kBigCap = 8192;     // one-warp-per-block table (<= 4096)
+constexpr int kBigCap = 8192;     // a block's table (<= 4096)
 constexpr int kRapWarps = 4;
+constexpr long long kSortProducts = 16384;  // rows with more are sorted (hub rows)
 
 __device__ __forceinline__ unsigned rap_hash(int key, unsigned mask) {
   return ((unsigned)key * 2654435761u >> 7) & mask;
@@ -129,8 +129,8 @@ __device__ __forceinline__ int warp_total(int v, int lane, int* start) {
   return __shfl_sync(0xffffffffu, incl, 31);
 }
 
-// A coarse row's products (r*a)*p in the reference's order, up to 32 at a time:
-// use(active, column, r*a, p).  The row is a chain of dependent loads (R's entry,
+// The products (r*a)*p of R's entries [r0, r1) in the reference's order, up to 32 at
+// a time: use(active, column, r*a, p).  The row is a chain of dependent loads (R's entry,
 // A's row bounds, A's entry, P's row bounds, P's entry), and a launch waits for its
 // longest row.  So R's entries are taken 32 at a time and their A entries as one
 // list of which each lane holds one, whatever rows they are from, and so for the P
@@ -140,7 +140,7 @@ __device__ __forceinline__ int warp_total(int v, int lane, int* start) {
 // 512 columns 412 -> 333, of up to 64 columns 130 -> 102; counting rows of 65 to
 // 512 products 224 -> 76).
 template <bool VAL, class F>
-__device__ __forceinline__ void rap_products(int ic, int lane, const int* __restrict__ ria,
+__device__ __forceinline__ void rap_products(int r0, int r1, int lane,
                                              const int* __restrict__ rja,
                                              const double* __restrict__ rval,
                                              const int* __restrict__ aia,
@@ -149,8 +149,7 @@ __device__ __forceinline__ void rap_products(int ic, int lane, const int* __rest
                                              const int* __restrict__ pia,
                                              const int* __restrict__ pja,
                                              const double* __restrict__ pval, F&& use) {
-  const int r1 = ria[ic + 1];
-  for (int kb = ria[ic]; kb < r1; kb += 32) {
+  for (int kb = r0; kb < r1; kb += 32) {
     int a0 = 0, alen = 0, astart;
     double r = 0.0;
     if (kb + lane < r1) {
@@ -224,7 +223,7 @@ __device__ int rap_count_row(int ic, Table t, int lane, const int* __restrict__ 
   __syncwarp();
   int cnt = 0;
   if (lane == 0) cnt += table_insert_atomic(t, ic);
-  rap_products<false>(ic, lane, ria, rja, nullptr, aia, aja, nullptr, pia, pja, nullptr,
+  rap_products<false>(ria[ic], ria[ic + 1], lane, rja, nullptr, aia, aja, nullptr, pia, pja, nullptr,
                       [&](bool act, int col, double, double) {
                         if (act) cnt += table_insert_atomic(t, col);
                       });
@@ -243,13 +242,23 @@ __device__ __forceinline__ int table_find_slot(Table t, int key) {
     h = (h + 1) & t.mask;
   }
 }
+// its place in the table, or -1
+__device__ __forceinline__ int table_at(Table t, int key) {
+  unsigned h = rap_hash(key, t.mask);
+  while (true) {
+    const int k = t.keys[h];
+    if (k == key) return (int)h;
+    if (k == -1) return -1;
+    h = (h + 1) & t.mask;
+  }
+}
 // insert a key known to be absent (lanes insert distinct keys concurrently)
-__device__ __forceinline__ void table_put(Table t, int key, int slot) {
+__device__ __forceinline__ int table_put(Table t, int key, int slot) {
   unsigned h = rap_hash(key, t.mask);
   while (true) {
     if (atomicCAS(&t.keys[h], -1, key) == -1) {
       t.slots[h] = slot;
-      return;
+      return (int)h;
     }
     h = (h + 1) & t.mask;
   }
@@ -279,7 +288,7 @@ __device__ void rap_fill_row(int ic, Table t, int lane, double* bval,
   // slot, numbered in order of first appearance); distinct columns proceed in
   // parallel
   rap_products<true>(
-      ic, lane, ria, rja, rval, aia, aja, aval, pia, pja, pval,
+      ria[ic], ria[ic + 1], lane, rja, rval, aia, aja, aval, pia, pja, pval,
       [&](bool act, int c, double ra, double p) {
         const double v = xmul(ra, p);
         bval[lane] = v;
@@ -350,7 +359,7 @@ k_rap_fill_small(const int* __restrict__ ria, const int* __restrict__ rja,
 }
 
 // ---------------- pass 1 kernels
-// class 0: per-warp shared table; class 1: one warp per block, big table;
+// class 0: per-warp shared table; class 1: a block with a big table;
 // class 2: global table (toff gives each listed row's table offset)
 __global__ void __launch_bounds__(32 * kRapWarps)
 k_rap_count_warp(const int* __restrict__ ria, const int* __restrict__ rja,
@@ -368,9 +377,10 @@ k_rap_count_warp(const int* __restrict__ ria, const int* __restrict__ rja,
 }
 
 // The rows with many products, a block each: a count does not depend on the order
-// of the insertions, so all threads share the row's table.  With a warp per row
-// the launch waited for its longest row (levels of a 1M-row network: 660 us a
-// call, now 294; the one with rows beyond shared tables 2,100 -> 680).
+// of the insertions, so all threads share the row's table and each warp walks a run
+// of R's entries (levels of a 1M-row network, us a call: a warp per row 660, a warp
+// per entry of R at a time 294, runs 127; the one with rows beyond shared tables
+// 2,100, 680, under 230).
 constexpr int kCountThreads = 256;
 __device__ int rap_count_block(int ic, Table t, const int* __restrict__ ria,
                                const int* __restrict__ rja, const int* __restrict__ aia,
@@ -383,22 +393,14 @@ __device__ int rap_count_block(int ic, Table t, const int* __restrict__ ria,
   __syncthreads();
   int cnt = 0;
   if (tid == 0) cnt += table_insert_atomic(t, ic);
-  const int lane = tid & 31, w = tid >> 5;
-  auto entry = [&](int k2) {
-    const int i2 = aja[k2];
-    for (int k3 = pia[i2]; k3 < pia[i2 + 1]; k3++) cnt += table_insert_atomic(t, pja[k3]);
-  };
-  // R's entries a warp each; rows of A that are long themselves take the block
-  for (int k1 = ria[ic] + w; k1 < ria[ic + 1]; k1 += kCountThreads / 32) {
-    const int i1 = rja[k1], a0 = aia[i1], a1 = aia[i1 + 1];
-    if (a1 - a0 > kCountThreads) continue;
-    for (int k2 = a0 + lane; k2 < a1; k2 += 32) entry(k2);
-  }
-  for (int k1 = ria[ic]; k1 < ria[ic + 1]; k1++) {
-    const int i1 = rja[k1], a0 = aia[i1], a1 = aia[i1 + 1];
-    if (a1 - a0 <= kCountThreads) continue;
-    for (int k2 = a0 + tid; k2 < a1; k2 += kCountThreads) entry(k2);
-  }
+  // a run of R's entries for each warp
+  const int r0 = ria[ic], w = tid >> 5;
+  const long long len = ria[ic + 1] - r0;
+  rap_products<false>(r0 + (int)(len * w / (kCountThreads / 32)),
+                      r0 + (int)(len * (w + 1) / (kCountThreads / 32)), tid & 31, rja, nullptr, aia,
+                      aja, nullptr, pia, pja, nullptr, [&](bool act, int col, double, double) {
+                        if (act) cnt += table_insert_atomic(t, col);
+                      });
   for (int off = 16; off > 0; off >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
   if ((tid & 31) == 0) atomicAdd(&total, cnt);
   __syncthreads();
@@ -439,8 +441,6 @@ k_rap_count_huge(const int* __restrict__ ria, const int* __restrict__ rja,
 // ---------------- pass 2 kernels
 constexpr size_t kWarpFillSmem =
     kRapWarps * (kWarpCap * 2 * sizeof(int) + (kWarpCap / 2 + 32) * sizeof(double));
-constexpr size_t kBigFillSmem =
-    kBigCap * 2 * sizeof(int) + (kBigCap / 2 + 32) * sizeof(double);
 constexpr size_t kBigCountSmem = kBigCap * sizeof(int);
 
 __device__ __forceinline__ void carve(unsigned char* base, int cap, Table* t, double** bval) {
@@ -471,22 +471,118 @@ k_rap_fill_warp(const int* __restrict__ ria, const int* __restrict__ rja,
   }
 }
 
-__global__ void __launch_bounds__(32)
-k_rap_fill_big(const int* __restrict__ ria, const int* __restrict__ rja,
-               const double* __restrict__ rval, const int* __restrict__ aia,
-               const int* __restrict__ aja, const double* __restrict__ aval,
-               const int* __restrict__ pia, const int* __restrict__ pja,
-               const double* __restrict__ pval, const int* __restrict__ rows, int m,
-               const int* __restrict__ cia, int* __restrict__ cja, double* __restrict__ cval) {
+// The rows with many products whose table fits, a block each.  A warp adds a row's
+// products 32 at a time at some 1,200 cycles (grouping the equal columns, finding
+// them, adding the longest group), and the launch waited for its longest row.  Here
+// every warp walks the row's products and takes the columns of its eighth of the
+// hash values, each still summed in stream order by one lane; positions of first
+// appearance, a bit each, give the columns' order at the end.  Filling the rows of
+// over 64 columns of a 1M-row network: 3.64 ms by warps, 2.99 with those over 1,024
+// products or 512 columns by blocks.
+constexpr int kBlockProducts = 1024;
+constexpr int kFillThreads = 256;
+constexpr int kFillWarps = kFillThreads / 32;
+constexpr int kPosWords = (int)(kSortProducts / 32);  // positions 0 .. kSortProducts - 1
+
+constexpr size_t block_fill_smem(int cap) {
+  return (size_t)cap * (sizeof(double) + 2 * sizeof(int)) +
+         kFillWarps * 64 * (sizeof(double) + 2 * sizeof(int)) + 2 * kPosWords * sizeof(int);
+}
+
+template <int CAP>
+__global__ void __launch_bounds__(kFillThreads)
+k_rap_fill_block(const int* __restrict__ ria, const int* __restrict__ rja,
+                 const double* __restrict__ rval, const int* __restrict__ aia,
+                 const int* __restrict__ aja, const double* __restrict__ aval,
+                 const int* __restrict__ pia, const int* __restrict__ pja,
+                 const double* __restrict__ pval, const int* __restrict__ rows, int m,
+                 const int* __restrict__ cia, int* __restrict__ cja, double* __restrict__ cval) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int lane = threadIdx.x & 31;
-  Table t;
-  double* bval;
-  carve(smem, kBigCap, &t, &bval);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  double* vals = (double*)smem;                        // by table position
+  double* qval = vals + CAP + w * 64;                  // the warp's products in waiting
+  int* keys = (int*)(vals + CAP + kFillWarps * 64);
+  int* first = keys + CAP;                             // position of first appearance
+  int* qcol = first + CAP + w * 64;
+  int* qpos = qcol + kFillWarps * 64;
+  unsigned* bits = (unsigned*)(first + CAP + 2 * kFillWarps * 64);
+  int* before = (int*)(bits + kPosWords);
+  const Table t{keys, first, vals, CAP - 1};
   for (int q = blockIdx.x; q < m; q += gridDim.x) {
     const int ic = rows[q];
-    rap_fill_row(ic, t, lane, bval, ria, rja, rval, aia, aja, aval, pia, pja, pval, cia[ic],
-                 cja, cval);
+    for (int e = tid; e < CAP; e += kFillThreads) keys[e] = -1;
+    for (int e = tid; e < kPosWords; e += kFillThreads) bits[e] = 0;
+    __syncthreads();
+    if (tid == 0) vals[table_put(t, ic, 0)] = 0.0;
+    __syncthreads();
+    int nq = 0, pos = 1;  // warp-uniform
+    auto add = [&](int cnt) {  // the first cnt <= 32 products in waiting
+      __syncwarp();
+      const bool act = lane < cnt;
+      const int col = act ? qcol[lane] : -1 - lane;
+      const unsigned grp = __match_any_sync(0xffffffffu, col);
+      if (act && (__ffs(grp) - 1 == lane)) {
+        int at = table_at(t, col);
+        double acc;
+        if (at < 0) {
+          at = table_put(t, col, qpos[lane]);
+          acc = qval[lane];
+        } else {
+          acc = xadd(vals[at], qval[lane]);
+        }
+        for (unsigned g = grp & (grp - 1); g; g &= g - 1) acc = xadd(acc, qval[__ffs(g) - 1]);
+        vals[at] = acc;
+      }
+      __syncwarp();
+    };
+    rap_products<true>(
+        ria[ic], ria[ic + 1], lane, rja, rval, aia, aja, aval, pia, pja, pval,
+        [&](bool act, int col, double ra, double p) {
+          const bool mine = act && (int)(((unsigned)col * 2654435761u) >> 29) == w;
+          const unsigned mm = __ballot_sync(0xffffffffu, mine);
+          if (mine) {
+            const int at = nq + __popc(mm & ((1u << lane) - 1u));
+            qcol[at] = col;
+            qval[at] = xmul(ra, p);
+            qpos[at] = pos + lane;
+          }
+          pos += __popc(__ballot_sync(0xffffffffu, act));
+          nq += __popc(mm);
+          if (nq >= 32) {
+            add(32);
+            nq -= 32;
+            if (lane < nq) {
+              qcol[lane] = qcol[lane + 32];
+              qval[lane] = qval[lane + 32];
+              qpos[lane] = qpos[lane + 32];
+            }
+            __syncwarp();
+          }
+        });
+    if (nq > 0) add(nq);
+    __syncthreads();
+    for (int e = tid; e < CAP; e += kFillThreads)
+      if (keys[e] != -1) atomicOr(&bits[first[e] >> 5], 1u << (first[e] & 31));
+    __syncthreads();
+    if (w == 0) {
+      int sum = 0;
+      for (int e0 = 0; e0 < kPosWords; e0 += 32) {
+        int start;
+        const int total = warp_total(__popc(bits[e0 + lane]), lane, &start);
+        before[e0 + lane] = sum + start;
+        sum += total;
+      }
+    }
+    __syncthreads();
+    const int cbase = cia[ic];
+    for (int e = tid; e < CAP; e += kFillThreads)
+      if (keys[e] != -1) {
+        const int p = first[e];
+        const int slot = before[p >> 5] + __popc(bits[p >> 5] & ((1u << (p & 31)) - 1u));
+        cja[cbase + slot] = keys[e];
+        cval[cbase + slot] = vals[e];
+      }
+    __syncthreads();
   }
 }
 
@@ -524,7 +620,6 @@ k_rap_fill_huge(const int* __restrict__ ria, const int* __restrict__ rja,
 // then sums them in that order (the first product assigned, the rest added,
 // exactly as the reference), and the columns are put back in order of first
 // appearance, which places the diagonal first.
-constexpr long long kSortProducts = 16384;
 constexpr long long kLongSeg = 256;  // segments longer than this are summed by a warp
 
 // products per (hub row, R entry) pair: sum over A row i1 of |P_i2|
@@ -910,8 +1005,10 @@ static void hub_finish(const int* rows, HubStream& H, CSR& Ac, cudaStream_t s) {
 
 // ---------------- classification helpers
 // class by a size estimate: 3 (<= kSmallCap/2), 0 (<= kWarpCap/2),
-// 1 (<= kBigCap/2), 2 (beyond)
-__global__ void k_rap_classify(const long long* __restrict__ est, int nc, int cap_limit,
+// 1 (<= kBigCap/2), 2 (beyond); of the rows of class 0 those with more than
+// kBlockProducts products (prod, if given) are class 4
+__global__ void k_rap_classify(const long long* __restrict__ est,
+                               const long long* __restrict__ prod, int nc, int cap_limit,
                                int* __restrict__ lists, int* __restrict__ counts) {
   // warp-aggregated appends: one atomic per class present in the warp
   const int lane = threadIdx.x & 31;
@@ -924,6 +1021,7 @@ __global__ void k_rap_classify(const long long* __restrict__ est, int nc, int ca
       if (e >= 0) {  // e < 0: handled elsewhere
         if (e > cap_limit) e = cap_limit;
         c = e <= kSmallCap / 2 ? 3 : (e <= kWarpCap / 2 ? 0 : (e <= kBigCap / 2 ? 1 : 2));
+        if (c == 0 && prod != nullptr && prod[ic] > kBlockProducts) c = 4;
       }
     }
     const unsigned grp = __match_any_sync(0xffffffffu, c);
@@ -966,17 +1064,18 @@ __global__ void k_i32_to_i64(const int* __restrict__ a, int n, long long* __rest
 }
 
 struct RapClasses {
-  DBuf<int> lists;  // 4 x nc
-  int count[4] = {0, 0, 0, 0};
+  DBuf<int> lists;  // 5 x nc
+  int count[5] = {0, 0, 0, 0, 0};
 };
 
-static void classify(const long long* est, int nc, RapClasses& rc, cudaStream_t s) {
-  rc.lists.alloc((size_t)4 * (nc > 0 ? nc : 1), s);
-  DBuf<int> cnt(4, s);
+static void classify(const long long* est, const long long* prod, int nc, RapClasses& rc,
+                     cudaStream_t s) {
+  rc.lists.alloc((size_t)5 * (nc > 0 ? nc : 1), s);
+  DBuf<int> cnt(5, s);
   cnt.zero();
   if (nc > 0)
-    BN_LAUNCH(k_rap_classify, grid_for(nc, 256), 256, 0, s, est, nc, nc, rc.lists.p, cnt.p);
-  cnt.download(rc.count, 4);
+    BN_LAUNCH(k_rap_classify, grid_for(nc, 256), 256, 0, s, est, prod, nc, nc, rc.lists.p, cnt.p);
+  cnt.download(rc.count, 5);
   BN_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -984,8 +1083,9 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
   const int nc = R.n;
   BN_CUDA(cudaFuncSetAttribute(k_rap_fill_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kWarpFillSmem));
-  BN_CUDA(cudaFuncSetAttribute(k_rap_fill_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kBigFillSmem));
+  BN_CUDA(cudaFuncSetAttribute(k_rap_fill_block<kBigCap>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)block_fill_smem(kBigCap)));
   BN_CUDA(cudaFuncSetAttribute(k_rap_count_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kBigCountSmem));
   DBuf<long long> ub(nc > 0 ? nc : 1, s), est(nc > 0 ? nc : 1, s);
@@ -1021,7 +1121,7 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
   }
   {
     RapClasses rc;
-    classify(est.p, nc, rc, s);
+    classify(est.p, nullptr, nc, rc, s);
     const int* L0 = rc.lists.p;
     const int* L1 = rc.lists.p + nc;
     const int* L2 = rc.lists.p + 2 * (size_t)nc;
@@ -1068,14 +1168,15 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
       BN_LAUNCH(k_rap_split_hubs, grid_for(nc, 256), 256, 0, s, ub.p, exact.p, nc, est.p, hub.p,
                 nh.p);
     RapClasses rc;
-    classify(est.p, nc, rc, s);
+    classify(est.p, ub.p, nc, rc, s);
     const int* L0 = rc.lists.p;
     const int* L1 = rc.lists.p + nc;
     const int* L2 = rc.lists.p + 2 * (size_t)nc;
     const int* L3 = rc.lists.p + 3 * (size_t)nc;
+    const int* L4 = rc.lists.p + 4 * (size_t)nc;
     if (trace_on())
-      fprintf(stderr, "[bn]     rap fill classes: small %d warp %d big %d huge %d hubs %d\n",
-              rc.count[3], rc.count[0], rc.count[1], rc.count[2], nhub);
+      fprintf(stderr, "[bn]     rap fill classes: small %d warp %d block %d big %d huge %d hubs %d\n",
+              rc.count[3], rc.count[0], rc.count[4], rc.count[1], rc.count[2], nhub);
     Phase ph_w("rap fill warp", s);
     if (rc.count[3])
       BN_LAUNCH(k_rap_fill_small, grid_for(rc.count[3], kSmallWarps, 64), 32 * kSmallWarps, 0, s,
@@ -1088,9 +1189,13 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
     ph_w.done();
     Phase ph_b("rap fill big", s);
     if (rc.count[1])
-      BN_LAUNCH(k_rap_fill_big, grid_for(rc.count[1], 1, 2), 32, kBigFillSmem, s, R.ia.p, R.ja.p,
-                R.val.p, A.ia.p, A.ja.p, A.val.p, P.ia.p, P.ja.p, P.val.p, L1, rc.count[1],
-                Ac.ia.p, Ac.ja.p, Ac.val.p);
+      BN_LAUNCH(k_rap_fill_block<kBigCap>, grid_for(rc.count[1], 1, 1), kFillThreads,
+                block_fill_smem(kBigCap), s, R.ia.p, R.ja.p, R.val.p, A.ia.p, A.ja.p, A.val.p,
+                P.ia.p, P.ja.p, P.val.p, L1, rc.count[1], Ac.ia.p, Ac.ja.p, Ac.val.p);
+    if (rc.count[4])
+      BN_LAUNCH(k_rap_fill_block<kWarpCap>, grid_for(rc.count[4], 1, 6), kFillThreads,
+                block_fill_smem(kWarpCap), s, R.ia.p, R.ja.p, R.val.p, A.ia.p, A.ja.p, A.val.p,
+                P.ia.p, P.ja.p, P.val.p, L4, rc.count[4], Ac.ia.p, Ac.ja.p, Ac.val.p);
     ph_b.done();
     Phase ph_h("rap fill huge", s);
     if (rc.count[2]) {

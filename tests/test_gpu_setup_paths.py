@@ -77,3 +77,40 @@ def test_rand_state_after_a_pmis_hierarchy(nodes):
     for _ in range(last):
         libc.rand()
     assert got == [libc.rand() for _ in range(3)]
+
+
+def test_rap_rows_of_every_class(oracle):
+    """Coarse rows of given numbers of products and of distinct columns, both sides of
+    each bound of the row classes, A rows of 0 to 3,000 entries among them."""
+    rng = np.random.default_rng(8)
+    # products without the diagonal's own, distinct columns
+    want = [(0, 1), (63, 64), (64, 40), (300, 65), (512, 500), (1023, 90), (1024, 90),
+            (1025, 512), (1025, 513), (4000, 20), (9000, 512), (16383, 512), (16383, 513),
+            (16383, 4096), (16383, 4097), (16384, 512), (16384, 3000)]
+    nc = 5000
+    R, Arows = [[] for _ in range(nc)], [[] for _ in range(nc)]
+    for ic, (products, width) in enumerate(want):
+        cols = np.r_[np.arange(min(width, products)), rng.integers(0, width, max(0, products - width))]
+        rng.shuffle(cols)
+        at = 0
+        while at < products:
+            m = int(rng.choice([0, 1, 3, 8, 33, 3000 if products > 10_000 else 5]))
+            R[ic].append(len(Arows))
+            Arows.append(cols[at:at + m])
+            at += m
+    nf = len(Arows)
+
+    def csr(rows):
+        ia = np.r_[0, np.cumsum([len(r) for r in rows])].astype(np.int32)
+        ja = np.concatenate([np.asarray(r, np.int32) for r in rows] + [np.zeros(0, np.int32)])
+        return ia, ja.astype(np.int32), rng.standard_normal(len(ja))
+
+    R, A = csr(R), csr(Arows)
+    P = csr([[i] if i < nc else [] for i in range(nf)])
+    ref_ = oracle.orc_rap(nc, nf, R, A, P)
+    out = amg.DcsrMat()
+    amg.load_library().dcsr_rap(C.byref(_dcsr(nc, nf, *R)), C.byref(_dcsr(nf, nf, *A)),
+                                C.byref(_dcsr(nf, nc, *P)), C.byref(out))
+    got = _out(out)
+    for j in range(3):
+        assert bits_equal(got[j], ref_[j])
