@@ -472,13 +472,16 @@ k_rap_fill_warp(const int* __restrict__ ria, const int* __restrict__ rja,
 }
 
 // The rows with many products whose table fits, a block each.  A warp adds a row's
-// products 32 at a time at some 1,200 cycles (grouping the equal columns, finding
-// them, adding the longest group), and the launch waited for its longest row.  Here
-// every warp walks the row's products and takes the columns of its eighth of the
-// hash values, each still summed in stream order by one lane; positions of first
-// appearance, a bit each, give the columns' order at the end.  Filling the rows of
-// over 64 columns of a 1M-row network: 3.64 ms by warps, 2.99 with those over 1,024
-// products or 512 columns by blocks.
+// products 32 at a time at some 1,200 cycles (a chain of instructions: finding the
+// entries, grouping the equal columns, looking them up), and the launch waited for
+// its longest row.  Here each warp forms the products of a run of R's entries (their
+// places follow from the counts per fine row, wprod) into a list in global memory
+// (192 KB, read back from L2), then takes from the whole list the columns of its
+// eighth of the hash values, each still summed in stream order by one lane;
+// positions of first appearance, a bit each, give the columns' order at the end.
+// Filling the rows of over 64 columns of a 1M-row network: 3.64 ms by warps, 2.99
+// with those over 1,024 products or 512 columns by blocks whose warps each formed
+// all products, 2.02 with runs.
 constexpr int kBlockProducts = 1024;
 constexpr int kFillThreads = 256;
 constexpr int kFillWarps = kFillThreads / 32;
@@ -495,10 +498,14 @@ k_rap_fill_block(const int* __restrict__ ria, const int* __restrict__ rja,
                  const double* __restrict__ rval, const int* __restrict__ aia,
                  const int* __restrict__ aja, const double* __restrict__ aval,
                  const int* __restrict__ pia, const int* __restrict__ pja,
-                 const double* __restrict__ pval, const int* __restrict__ rows, int m,
+                 const double* __restrict__ pval, const long long* __restrict__ wprod,
+                 const long long* __restrict__ ub, double* __restrict__ sval_all,
+                 int* __restrict__ scol_all, const int* __restrict__ rows, int m,
                  const int* __restrict__ cia, int* __restrict__ cja, double* __restrict__ cval) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  double* sval = sval_all + (size_t)blockIdx.x * kSortProducts;
+  int* scol = scol_all + (size_t)blockIdx.x * kSortProducts;
   double* vals = (double*)smem;                        // by table position
   double* qval = vals + CAP + w * 64;                  // the warp's products in waiting
   int* keys = (int*)(vals + CAP + kFillWarps * 64);
@@ -515,7 +522,36 @@ k_rap_fill_block(const int* __restrict__ ria, const int* __restrict__ rja,
     __syncthreads();
     if (tid == 0) vals[table_put(t, ic, 0)] = 0.0;
     __syncthreads();
-    int nq = 0, pos = 1;  // warp-uniform
+    // the warp's run of R's entries: those whose products start in its eighth
+    const int total = (int)(ub[ic] - 1), lo = (int)((long long)total * w / kFillWarps),
+              hi = (int)((long long)total * (w + 1) / kFillWarps);
+    int ra = -1, rb = -1, pos = 0, sum = 0;  // warp-uniform
+    for (int kb = ria[ic], r1 = ria[ic + 1]; kb < r1 && rb < 0; kb += 32) {
+      const int len = kb + lane < r1 ? (int)wprod[rja[kb + lane]] : 0;
+      int start;
+      const int t32 = warp_total(len, lane, &start);
+      start += sum;
+      const unsigned in = __ballot_sync(0xffffffffu, kb + lane < r1 && start >= lo);
+      const unsigned out = __ballot_sync(0xffffffffu, kb + lane < r1 && start >= hi);
+      if (ra < 0 && in) {
+        ra = kb + __ffs(in) - 1;
+        pos = __shfl_sync(0xffffffffu, start, __ffs(in) - 1);
+      }
+      if (out && w + 1 < kFillWarps) rb = kb + __ffs(out) - 1;
+      sum += t32;
+    }
+    if (rb < 0) rb = ria[ic + 1];
+    if (ra < 0) ra = rb;
+    rap_products<true>(ra, rb, lane, rja, rval, aia, aja, aval, pia, pja, pval,
+                       [&](bool act, int col, double r, double p) {
+                         if (act) {
+                           scol[pos + lane] = col;
+                           sval[pos + lane] = xmul(r, p);
+                         }
+                         pos += __popc(__ballot_sync(0xffffffffu, act));
+                       });
+    __syncthreads();
+    int nq = 0;  // warp-uniform
     auto add = [&](int cnt) {  // the first cnt <= 32 products in waiting
       __syncwarp();
       const bool act = lane < cnt;
@@ -535,30 +571,40 @@ k_rap_fill_block(const int* __restrict__ ria, const int* __restrict__ rja,
       }
       __syncwarp();
     };
-    rap_products<true>(
-        ria[ic], ria[ic + 1], lane, rja, rval, aia, aja, aval, pia, pja, pval,
-        [&](bool act, int col, double ra, double p) {
-          const bool mine = act && (int)(((unsigned)col * 2654435761u) >> 29) == w;
-          const unsigned mm = __ballot_sync(0xffffffffu, mine);
-          if (mine) {
-            const int at = nq + __popc(mm & ((1u << lane) - 1u));
-            qcol[at] = col;
-            qval[at] = xmul(ra, p);
-            qpos[at] = pos + lane;
+    for (int q0 = 0; q0 < total; q0 += 128) {
+      int col[4];
+      double val[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int at = q0 + 32 * u + lane;
+        col[u] = at < total ? scol[at] : 0;
+        val[u] = at < total ? sval[at] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int at = q0 + 32 * u + lane;
+        const bool mine =
+            at < total && (int)(((unsigned)col[u] * 2654435761u) >> 29) == w;
+        const unsigned mm = __ballot_sync(0xffffffffu, mine);
+        if (mine) {
+          const int k = nq + __popc(mm & ((1u << lane) - 1u));
+          qcol[k] = col[u];
+          qval[k] = val[u];
+          qpos[k] = at + 1;
+        }
+        nq += __popc(mm);
+        if (nq >= 32) {
+          add(32);
+          nq -= 32;
+          if (lane < nq) {
+            qcol[lane] = qcol[lane + 32];
+            qval[lane] = qval[lane + 32];
+            qpos[lane] = qpos[lane + 32];
           }
-          pos += __popc(__ballot_sync(0xffffffffu, act));
-          nq += __popc(mm);
-          if (nq >= 32) {
-            add(32);
-            nq -= 32;
-            if (lane < nq) {
-              qcol[lane] = qcol[lane + 32];
-              qval[lane] = qval[lane + 32];
-              qpos[lane] = qpos[lane + 32];
-            }
-            __syncwarp();
-          }
-        });
+          __syncwarp();
+        }
+      }
+    }
     if (nq > 0) add(nq);
     __syncthreads();
     for (int e = tid; e < CAP; e += kFillThreads)
@@ -1093,8 +1139,8 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
   cnt.zero();
   nh.zero();
   Phase ph_bound("rap bound", s);
+  DBuf<long long> w(A.n > 0 ? A.n : 1, s);
   if (nc > 0) {
-    DBuf<long long> w(A.n > 0 ? A.n : 1, s);
     if (A.n > 0)
       BN_LAUNCH(k_fine_weights, grid_for((long long)A.n * 32, 256, 16), 256, 0, s, A.ia.p,
                 A.ja.p, P.ia.p, A.n, w.p);
@@ -1188,14 +1234,20 @@ void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s) {
                 P.ja.p, P.val.p, L0, rc.count[0], Ac.ia.p, Ac.ja.p, Ac.val.p);
     ph_w.done();
     Phase ph_b("rap fill big", s);
-    if (rc.count[1])
-      BN_LAUNCH(k_rap_fill_block<kBigCap>, grid_for(rc.count[1], 1, 1), kFillThreads,
-                block_fill_smem(kBigCap), s, R.ia.p, R.ja.p, R.val.p, A.ia.p, A.ja.p, A.val.p,
-                P.ia.p, P.ja.p, P.val.p, L1, rc.count[1], Ac.ia.p, Ac.ja.p, Ac.val.p);
-    if (rc.count[4])
-      BN_LAUNCH(k_rap_fill_block<kWarpCap>, grid_for(rc.count[4], 1, 6), kFillThreads,
-                block_fill_smem(kWarpCap), s, R.ia.p, R.ja.p, R.val.p, A.ia.p, A.ja.p, A.val.p,
-                P.ia.p, P.ja.p, P.val.p, L4, rc.count[4], Ac.ia.p, Ac.ja.p, Ac.val.p);
+    if (rc.count[1] + rc.count[4]) {
+      const int g1 = grid_for(rc.count[1], 1, 1), g4 = grid_for(rc.count[4], 1, 2);
+      const size_t stream = (size_t)(g1 > g4 ? g1 : g4) * kSortProducts;
+      DBuf<double> sval(stream, s);
+      DBuf<int> scol(stream, s);
+      if (rc.count[1])
+        BN_LAUNCH(k_rap_fill_block<kBigCap>, g1, kFillThreads, block_fill_smem(kBigCap), s, R.ia.p,
+                  R.ja.p, R.val.p, A.ia.p, A.ja.p, A.val.p, P.ia.p, P.ja.p, P.val.p, w.p, ub.p,
+                  sval.p, scol.p, L1, rc.count[1], Ac.ia.p, Ac.ja.p, Ac.val.p);
+      if (rc.count[4])
+        BN_LAUNCH(k_rap_fill_block<kWarpCap>, g4, kFillThreads, block_fill_smem(kWarpCap), s,
+                  R.ia.p, R.ja.p, R.val.p, A.ia.p, A.ja.p, A.val.p, P.ia.p, P.ja.p, P.val.p, w.p,
+                  ub.p, sval.p, scol.p, L4, rc.count[4], Ac.ia.p, Ac.ja.p, Ac.val.p);
+    }
     ph_b.done();
     Phase ph_h("rap fill huge", s);
     if (rc.count[2]) {
