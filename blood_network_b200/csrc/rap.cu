@@ -89,25 +89,6 @@ __global__ void k_rap_bound_w(const int* __restrict__ ria, const int* __restrict
   }
 }
 
-__global__ void k_rap_bound(const int* __restrict__ ria, const int* __restrict__ rja,
-                            const int* __restrict__ aia, const int* __restrict__ aja,
-                            const int* __restrict__ pia, int nc, long long* __restrict__ ub) {
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int ic = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ic < nc; ic += warps) {
-    long long b = 0;
-    for (int k1 = ria[ic]; k1 < ria[ic + 1]; k1++) {
-      int i1 = rja[k1];
-      for (int k2 = aia[i1] + lane; k2 < aia[i1 + 1]; k2 += 32) {
-        int i2 = aja[k2];
-        b += pia[i2 + 1] - pia[i2];
-      }
-    }
-    for (int off = 16; off > 0; off >>= 1) b += __shfl_xor_sync(0xffffffffu, b, off);
-    if (lane == 0) ub[ic] = 1 + b;
-  }
-}
-
 // lane of the entry e, given where each lane's entries start (ascending; a lane
 // without entries starts where the next one does)
 __device__ __forceinline__ int entry_lane(int start, int e) {
