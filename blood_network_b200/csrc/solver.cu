@@ -313,6 +313,7 @@ void Solver::drop_graphs() {
 void Solver::choose_tail() {
   const int nl = (int)lv.size();
   tail_l0 = nl;
+  tail_nu = opt.nu;
   const char* e = getenv("BN_TAIL");  // 0: every level on launches of its own
   if ((e && atoi(e) == 0) || nl < 2 || lv[nl - 1]->A.n > kTailDenseMax || lv[nl - 1]->A.n == 0) return;
   if (opt.smoother != SMOOTHER_CF_GS && opt.smoother != SMOOTHER_GS) return;
@@ -321,7 +322,7 @@ void Solver::choose_tail() {
   for (int l = nl - 2; l >= 0; l--) {
     const Level& L = *lv[l];
     if (L.gs_rows.n == 0 || L.A.n == 0 || L.A.n > kTailRows || L.A.nnz > kTailNnz) break;
-    ops += 2 * ((long long)L.cptr.size() - 1) * opt.nu + 5;
+    ops += 2 * ((long long)L.cptr.size() - 1) * tail_nu + 5;
     if (ops > kTailMaxOps) break;
     tail_l0 = l;
   }
@@ -407,7 +408,7 @@ void Solver::ensure_tail() {
       coarsest();
     } else {
       Level& L = *lv[l];
-      for (int k = 0; k < opt.nu; k++) sweep(l, true, k == 0);
+      for (int k = 0; k < tail_nu; k++) sweep(l, true, k == 0);
       add(TK_RES, l, &L.Ap, &L.A32, 0, L.A.n, vb(l), vx(l), vr(l), TT_B_IS_B | TT_X_IS_X);
       add(TK_Y, l, &L.Rp, &L.R32, 0, L.Rp.n, nullptr, vr(l), vb(l + 1), 0);
       back(l + 1);
@@ -424,7 +425,7 @@ void Solver::ensure_tail() {
       add(TK_Y, l, &L.Rp, &L.R32, 0, L.Rp.n, nullptr, vb(l), vb(l + 1), TT_X_IS_B);
       fwd(l + 1);
       add(TK_Y, l, &L.Pp, &L.P32, 0, L.A.n, nullptr, vx(l + 1), vx(l), TT_Y_IS_X);
-      for (int k = 0; k < opt.nu; k++) sweep(l, false, false);
+      for (int k = 0; k < tail_nu; k++) sweep(l, false, false);
     }
     P.fwd[l - tail_l0].y = (int)ops.size();
   };
@@ -1154,7 +1155,7 @@ void Solver::smooth(int l, const T* bb, T* xl, bool forward) {
 template <class T>
 void Solver::backslash(int l, const T* bb, T* xl, bool zero_guess) {
   const int nl = (int)lv.size();
-  if (zero_guess && l >= tail_l0) {
+  if (zero_guess && whole_tail(l)) {
     ensure_tail<T>();
     const int2 q = tail<T>().back[l - tail_l0];
     tail_run<T>(tail<T>().ops.p, q.x, q.y, l, bb, xl, tail_nblk, s);
@@ -1219,7 +1220,7 @@ void Solver::backslash(int l, const T* bb, T* xl, bool zero_guess) {
 template <class T>
 void Solver::fwdslash(int l, const T* bb, T* xl) {
   const int nl = (int)lv.size();
-  if (l >= tail_l0) {
+  if (whole_tail(l)) {
     ensure_tail<T>();
     const int2 q = tail<T>().fwd[l - tail_l0];
     tail_run<T>(tail<T>().ops.p, q.x, q.y, l, bb, xl, tail_nblk, s);

@@ -133,8 +133,12 @@ struct Solver {
   void build_solve_layout();
   // The coarse tail: levels tail_l0 .. coarsest (tail_l0 = number of levels:
   // none).  Its programs hold the vectors' addresses, so they go with the
-  // graphs (drop_graphs) and are made again before the next use.
-  int tail_l0 = 0, tail_nblk = 0;
+  // graphs (drop_graphs) and are made again before the next use.  The sweeps of
+  // its backslash and fwdslash are those of tail_nu, the handle's own number;
+  // calls that ask for another (amg_backslash and so on take one each) run its
+  // levels by single sweeps, which serve any number, and launches for the rest.
+  int tail_l0 = 0, tail_nblk = 0, tail_nu = 1;
+  bool whole_tail(int l) const { return l >= tail_l0 && opt.nu == tail_nu; }
   Tail<double> tail64;
   Tail<float> tail32;
   template <class T> Tail<T>& tail() {
