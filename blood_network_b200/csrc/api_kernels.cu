@@ -107,6 +107,19 @@ BN_API void rs_standard_interpolation_sparsity(const dcsr_mat* S, const int* cf,
   });
 }
 
+// A solver's matrices hold a column once per row (it refuses others); a
+// caller's need not.  Columns are points, so both matrices are n x n.
+static bool distinct_rows(const dcsr_mat* A, CSR& dA, const dcsr_mat* S, CSR& dS,
+                          cudaStream_t s) {
+  BN_REQUIRE(A->ia[A->row] <= A->nnz && S->ia[S->row] <= S->nnz, BN_ERR_ARG,
+             "row pointers beyond the entries");
+  dA.m = dA.n;
+  dS.m = dS.n;
+  dA.nnz = A->ia[A->row];  // entries of the rows; the arrays may be longer
+  dS.nnz = S->ia[S->row];
+  return distinct_columns(dA, dS, s);
+}
+
 BN_API void rs_standard_interpolation_values(const dcsr_mat* A, const dcsr_mat* S, const int* cf,
                                              dcsr_mat* P) {
   api_call([&]() {
@@ -118,7 +131,7 @@ BN_API void rs_standard_interpolation_values(const dcsr_mat* A, const dcsr_mat* 
     to_device(P, dP, s);
     DBuf<int> dcf(n > 0 ? n : 1, s);
     dcf.upload(cf, n);
-    interpolation_values(dA, dS, dcf.p, dP, s);
+    interpolation_values(dA, dS, dcf.p, dP, s, distinct_rows(A, dA, S, dS, s));
     dP.val.download(P->val, P->nnz);
     BN_CUDA(cudaStreamSynchronize(s));
   });
@@ -136,7 +149,7 @@ BN_API void rs_standard_interpolation(const dcsr_mat* A, const dcsr_mat* S, cons
     dcf.upload(cf, n);
     int nc = 0;
     for (int i = 0; i < n; i++) nc += (cf[i] == 1);
-    interpolation(dA, dS, dcf.p, nc, dP, s);
+    interpolation(dA, dS, dcf.p, nc, dP, s, distinct_rows(A, dA, S, dS, s));
     to_host(dP, P, s);
   });
 }

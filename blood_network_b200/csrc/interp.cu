@@ -574,9 +574,75 @@ __global__ void k_interp_values(const int* __restrict__ aia, const int* __restri
   }
 }
 
-void interpolation_values(const CSR& A, const CSR& S, const int* cf, CSR& P, cudaStream_t s) {
+// flag[0] = 1: a row of at most kTwiceRow entries holds a column twice;
+// flag[1] = 1: there are longer rows.  A warp per row, all pairs (1M-row network,
+// both matrices: 0.4 ms of the call's 10; all rows by the transpose 3).
+constexpr int kTwiceRow = 512;
+__global__ void k_twice(const int* __restrict__ ia, const int* __restrict__ ja, int n,
+                        int* __restrict__ flag) {
+  const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const int k0 = ia[i], k1 = ia[i + 1];
+    if (k1 - k0 > kTwiceRow) {
+      if (lane == 0) flag[1] = 1;
+      continue;
+    }
+    bool twice = false;
+    for (int base = k0; base < k1; base += 32) {
+      const int j = base + lane < k1 ? ja[base + lane] : -1 - lane;  // columns are not negative
+      twice |= __popc(__match_any_sync(0xffffffffu, j)) > 1;
+      for (int k = k0; k < base; k++) twice |= ja[k] == j;
+    }
+    if (twice) flag[0] = 1;
+  }
+}
+// The long rows, in the transpose: a column's rows stand there in increasing
+// order, so a row that holds the column twice is there twice in a row.
+__global__ void k_twice_t(const int* __restrict__ tia, const int* __restrict__ tja, int m,
+                          int* __restrict__ flag) {
+  const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  for (int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < m; j += warps)
+    for (int k = tia[j] + 1 + lane; k < tia[j + 1]; k += 32)
+      if (tja[k] == tja[k - 1]) flag[0] = 1;
+}
+
+bool distinct_columns(const CSR& A, const CSR& S, cudaStream_t s) {
+  const CSR* ms[2] = {&A, &S};
+  DBuf<int> flags(4, s);
+  flags.zero();
+  for (int q = 0; q < 2; q++)
+    if (ms[q]->n > 0)
+      BN_LAUNCH(k_twice, grid_for((long long)ms[q]->n * 32, 256, 16), 256, 0, s, ms[q]->ia.p,
+                ms[q]->ja.p, ms[q]->n, flags.p + 2 * q);
+  int h[4];
+  flags.download(h, 4);
+  BN_CUDA(cudaStreamSynchronize(s));
+  if (h[0] || h[2]) return false;
+  for (int q = 0; q < 2; q++) {
+    if (!h[2 * q + 1]) continue;
+    CSR T;
+    transpose(*ms[q], T, s, false);
+    BN_LAUNCH(k_twice_t, grid_for((long long)T.n * 32, 256, 16), 256, 0, s, T.ia.p, T.ja.p, T.n,
+              flags.p);
+    if (read_scalar(flags.p, s)) return false;
+  }
+  return true;
+}
+
+void interpolation_values(const CSR& A, const CSR& S, const int* cf, CSR& P, cudaStream_t s,
+                          bool distinct) {
   if (A.n == 0) return;
   const int n = A.n;
+  if (!distinct) {
+    // The warp and block kernels and the hub tables count on one entry per
+    // column (they add a neighbour's entries in parallel and keep at most one
+    // per strong point); a thread per row takes the entries as they come.
+    DBuf<unsigned char> wide(n, s);
+    wide.zero();
+    BN_LAUNCH(k_interp_values, grid_for(n, 128), 128, 0, s, A.ia.p, A.ja.p, A.val.p, S.ia.p,
+              S.ja.p, cf, n, wide.p, P.ia.p, P.val.p, nullptr, nullptr, nullptr, nullptr);
+    return;
+  }
   DBuf<int> hubidx(n, s), hubrows(n, s), ctr(2, s);
   ctr.zero();
   BN_LAUNCH(k_hub_mark, grid_for(n, 256), 256, 0, s, A.ia.p, n, hubidx.p, hubrows.p, ctr.p);
@@ -634,9 +700,9 @@ void interpolation_pattern(const CSR& S, const int* cf, int n_coarse, CSR& P, cu
 }
 
 void interpolation(const CSR& A, const CSR& S, const int* cf, int n_coarse, CSR& P,
-                   cudaStream_t s) {
+                   cudaStream_t s, bool distinct) {
   interpolation_pattern(S, cf, n_coarse, P, s);
-  interpolation_values(A, S, cf, P, s);
+  interpolation_values(A, S, cf, P, s, distinct);
 }
 
 }  // namespace bn
