@@ -131,12 +131,11 @@ __device__ __forceinline__ int hub_find(const int* __restrict__ keys, const int*
 // F rows with more than kWarpRow entries of A (and at most kInterpMaxC
 // strong points) are evaluated by a warp.  The operations and their order
 // are those of the thread-per-row kernel: the lanes classify A's entries and
-// locate the strong C points, one lane adds the weak entries in row order,
-// the strong F neighbours are taken from S_i (the same entries of A in the
-// same order, S holding A's values), the entries of each neighbour's row
-// that lie in C_i are collected in row order and one lane sums the
-// denominator in that order; each slot of P's row receives its terms in the
-// same sequence as in the thread kernel.
+// locate the strong points, one lane adds the weak entries in row order, the
+// strong F neighbours are taken in the order of their entries of A, the
+// entries of each neighbour's row that lie in C_i are collected in row order
+// and one lane sums the denominator in that order; each slot of P's row
+// receives its terms in the same sequence as in the thread kernel.
 constexpr int kWarpRow = 32;
 // ... and so are shorter ones whose strong F neighbours' rows hold more than
 // kWarpWalk entries together: a thread walks them twice, a slot search per
@@ -331,6 +330,7 @@ k_interp_values_block(const int* __restrict__ aia, const int* __restrict__ aja,
 }
 
 constexpr int kInterpWarps = 4;
+constexpr int kNoPos = 0x7fffffff;
 
 __global__ void __launch_bounds__(32 * kInterpWarps)
 k_interp_values_warp(const int* __restrict__ aia, const int* __restrict__ aja,
@@ -341,7 +341,8 @@ k_interp_values_warp(const int* __restrict__ aia, const int* __restrict__ aja,
                      const int* __restrict__ hubidx, const int* __restrict__ hoff,
                      const int* __restrict__ hkeys, const int* __restrict__ hvals) {
   __shared__ int s_col[kInterpWarps][32];   // S_i columns, S order
-  __shared__ int s_slot[kInterpWarps][32];  // slot in P's row (C) or -1 (F)
+  __shared__ int s_slot[kInterpWarps][32];  // slot in P's row (C), -1 (F) or -2 (neither)
+  __shared__ int s_pos[kInterpWarps][32];   // F: its entry of A
   __shared__ int s_cm[kInterpWarps][32];    // C_i columns by slot
   __shared__ double s_buf[kInterpWarps][32];
   __shared__ double s_af[kInterpWarps][32];  // a_ik of A (not S) for the strong F points
@@ -350,6 +351,7 @@ k_interp_values_warp(const int* __restrict__ aia, const int* __restrict__ aja,
   const unsigned lt = (1u << lane) - 1u;
   int* col = s_col[w];
   int* slt = s_slot[w];
+  int* pos = s_pos[w];
   int* cm = s_cm[w];
   double* buf = s_buf[w];
   double* af = s_af[w];
@@ -361,19 +363,21 @@ k_interp_values_warp(const int* __restrict__ aia, const int* __restrict__ aja,
     const int p0 = pia[i];
     const int s0 = sia[i], ns = sia[i + 1] - s0;
     // strong points of i and their slots
-    int q = -1, isc = 0;
+    int q = -1, kind = 0;
     if (lane < ns) {
       q = sja[s0 + lane];
-      isc = (cf[q] == 1);
+      kind = cf[q];
     }
+    const bool isc = kind == 1;
     const unsigned cmask = __ballot_sync(0xffffffffu, isc);
     const int nc = __popc(cmask);
     if (lane < ns) {
       col[lane] = q;
-      slt[lane] = isc ? __popc(cmask & lt) : -1;
+      slt[lane] = isc ? __popc(cmask & lt) : kind == -1 ? -1 : -2;
       if (isc) cm[__popc(cmask & lt)] = q;
     }
     if (lane < nc) pval[p0 + lane] = 0.0;
+    pos[lane] = kNoPos;
     __syncwarp();
     // A_i: diagonal, direct C terms, weak sum (one lane, row order)
     double diag = 0.0, weak = 0.0;
@@ -391,9 +395,12 @@ k_interp_values_warp(const int* __restrict__ aia, const int* __restrict__ aja,
           int at = -1;
           for (int t = 0; t < ns; t++)
             if (col[t] == j) { at = t; break; }
-          if (at < 0) cls = 1;
+          if (at < 0 || slt[at] == -2) cls = 1;
           else if (slt[at] >= 0) pval[p0 + slt[at]] = xadd(pval[p0 + slt[at]], a);  // once per slot
-          else af[at] = a;  // strong F point: its a_ik, from A (a value refresh keeps S's old values)
+          else {  // strong F point: its a_ik, from A (a value refresh keeps S's old values)
+            af[at] = a;
+            pos[at] = k;
+          }
         }
       }
       const unsigned wm = __ballot_sync(0xffffffffu, cls == 1);
@@ -408,9 +415,14 @@ k_interp_values_warp(const int* __restrict__ aia, const int* __restrict__ aja,
       __syncwarp();
     }
     double diag_hat = xadd(diag, weak);  // meaningful on lane 0
-    // strong F neighbours in S order (= A order)
-    for (int t = 0; t < ns; t++) {
-      if (slt[t] >= 0) continue;
+    // strong F neighbours in A order; a strong point without an entry of A (a
+    // caller's S, or values updated on another pattern) has no part in it
+    const int mine = pos[lane];
+    for (int last = -1;;) {
+      const int next = __reduce_min_sync(0xffffffffu, mine > last ? mine : kNoPos);
+      if (next == kNoPos) break;
+      last = next;
+      const int t = __ffs(__ballot_sync(0xffffffffu, mine == next)) - 1;
       const int kk = col[t];
       const double a_ik = af[t];
       const int h = hubidx ? hubidx[kk] : -1;

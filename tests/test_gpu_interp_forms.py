@@ -74,3 +74,26 @@ def test_strong_points_held_twice(oracle):
         a[2][:] = np.bincount(np.unique(rows * n + a[1], return_inverse=True)[1], a[2])[
             np.unique(rows * n + a[1], return_inverse=True)[1]]
     assert np.array_equal(P[2], want[2])
+
+
+@pytest.mark.parametrize("form", ["order", "extra", "diagonal", "undecided"])
+def test_strong_points_unlike_the_row(oracle, form):
+    """Strong points in another order than A's entries, some that A has no entry
+    for, the point itself among them, points that are neither C nor F."""
+    n, A, rng, cf = _problem(7)
+
+    def other(i, c, v):
+        if form == "extra":
+            more = np.setdiff1d(rng.integers(0, 1600, 3), np.r_[c, A[1][A[0][i]:A[0][i + 1]]])
+            c, v = np.r_[c, more], np.r_[v, rng.standard_normal(len(more))]
+        if form == "diagonal":
+            c, v = np.r_[c, i], np.r_[v, 1.0]
+        at = rng.permutation(len(c))
+        return c[at], v[at]
+
+    S = _rows(*oracle.orc_strength(n, *A, 0.25)[0], other)
+    if form == "undecided":
+        cf[rng.random(n) < 0.2] = 0
+    P, want = _interp(n, A, S, cf), oracle.orc_interp(n, A, S, cf)
+    for a, b in zip(P, want):
+        assert bits_equal(a, b)
