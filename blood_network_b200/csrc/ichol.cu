@@ -995,6 +995,8 @@ void IChol::finish(const int* aia, const int* aja, const double* aval, bool nume
   ph_lay.done();
   {
     Phase ph("ichol values", s);
+    if (!want_f32)  // of the factor before, if any: made anew when asked for
+      for (auto* v : {&fval32, &bval32, &fdiag32, &bdiag32}) *v = DBuf<float>();
     refresh_values();
     remap(nullptr, s);
   }

@@ -2142,7 +2142,11 @@ BN_API int amg_solver_bench_kernel(void* h, int which, int precision, int reps, 
     BN_CUDA(cudaSetDevice(S->device));
     const bool f32 = precision == 1;
     if (f32 && !S->f32_ready) {
-      if (!S->ic.fval32.n) { S->ic.want_f32 = true; S->ic.refresh_values(); }
+      if (!S->ic.fval32.n) {
+        S->ic.want_f32 = true;
+        S->ic.refresh_values();
+        S->drop_graphs();  // they hold the values' addresses
+      }
       S->prepare_f32();
     }
     if (f32 && !S->g32.n) {
