@@ -485,6 +485,17 @@ void IChol::own_values(cudaStream_t s) {
   }
 }
 
+// After a change of want_f32: the values in that precision, where the schedule
+// (made for the precision at the time) serves it and does not have them yet.
+void IChol::own_want(cudaStream_t s) {
+  const size_t bytes = want_f32 ? sizeof(float) : sizeof(double);
+  if (own_blocks == 0 || (want_f32 ? of.val32.n : of.val.n) > 0) return;
+  if ((size_t)own_rows * bytes > (size_t)own_limit ||
+      n > (long long)own_blocks * (want_f32 ? kOwnRows32 : kOwnRows64))
+    return;
+  own_values(s);
+}
+
 // One sweep; out holds the pending pattern everywhere.
 template <class T>
 void run_tri_own(const IChol& ic, bool forward, const T* in, T* out, T* clear, WaitCtl wc,

@@ -119,6 +119,7 @@ struct IChol {
   bool own_few = false;           // fewer blocks than SMs: smaller blocks
   void own_build(const int* inv, cudaStream_t s);
   void own_values(cudaStream_t s);
+  void own_want(cudaStream_t s);
   template <class T> bool own_ready() const;
   DBuf<int> fia, fja, fsrc; // forward rows (level order)
   DBuf<int> bia, bja, bsrc; // backward rows (reverse level order)

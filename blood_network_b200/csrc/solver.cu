@@ -928,6 +928,7 @@ void Solver::build_solve_layout() {
     analyze_rows(Aownp, layOwn, s);
     if (coloured_level(0)) order_tiles(Aownp.n, lv[0]->perm.p, layOwn, s);
   }
+  ic.want_f32 = (opt.precision == AMG_PREC_MIXED);  // a timing may have asked for FP32
   ic.remap(lv[0]->inv.p, s);
   f32_ready = false;
 }
@@ -1987,14 +1988,13 @@ BN_API int amg_solver_set_precision(void* h, int precision) {
                "unknown precision");
     BN_CUDA(cudaSetDevice(S->device));
     S->opt.precision = precision;
+    S->ic.want_f32 = precision == AMG_PREC_MIXED;
     if (precision == AMG_PREC_MIXED) {
-      if (!S->ic.fval32.n) {
-        S->ic.want_f32 = true;
-        S->ic.refresh_values();
-      }
+      if (!S->ic.fval32.n) S->ic.refresh_values();
       S->prepare_f32();
       S->alloc_vectors();
     }
+    S->ic.own_want(S->s);
     S->drop_graphs();
     return 0;
   }, bn::BN_ERR_ARG);

@@ -64,3 +64,47 @@ def test_fp32_timing_between_fp64_solves():
     other.close()
     s.close()
     assert x[1] == y[1] and x[0].tobytes() == y[0].tobytes()
+
+
+def _sweep_kernels(s, g):
+    """Names of the IC(0) sweep kernels of one preconditioner application."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        x = s.precond(g)
+        torch.cuda.synchronize()
+    return x, {e.name for e in p.events() if "k_tri_" in e.name}
+
+
+def test_owner_sweeps_in_the_precision_at_hand():
+    """The sweeps that keep rows by their blocks serve a handle in either precision,
+    whichever it was made in, and after a new smoother or new values; the results
+    are the chunked sweeps' bits, as in a handle made in that precision."""
+    n, ia, ja, val = VASCULAR
+    g = np.random.default_rng(3).standard_normal(n)
+    want = {}
+    for p in (amg.PREC_FP64, amg.PREC_MIXED):
+        s = amg.AMGSolver(n, ia, ja, val, min_size=200, precision=p)
+        want[p] = s.precond(g).tobytes()
+        s.close()
+
+    def check(s, p):
+        x, names = _sweep_kernels(s, g)
+        assert x.tobytes() == want[p]
+        kind = "k_tri_own<double" if p == amg.PREC_FP64 else "k_tri_own<float"
+        assert names and all(kind in m for m in names), names
+
+    for first, second in ((amg.PREC_MIXED, amg.PREC_FP64), (amg.PREC_FP64, amg.PREC_MIXED)):
+        s = amg.AMGSolver(n, ia, ja, val, min_size=200, precision=first)
+        check(s, first)
+        s.set_precision(second)
+        check(s, second)
+        s.set_smoother(amg.SMOOTHER_GS)
+        s.set_smoother(amg.SMOOTHER_CF_GS)
+        check(s, second)
+        s.update(ia, ja, val)
+        s.set_precision(first)
+        check(s, first)
+        s.bench_kernel(3, precision=1, reps=1)
+        check(s, first)
+        s.close()
