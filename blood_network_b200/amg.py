@@ -147,6 +147,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "ichol_free": (None, [C.POINTER(IcholFactor)]),
         "ichol_solve_noalloc": (i, [i, vp, vp, vp, vp, vp, vp]),
         "amg_debug_wait_timeout": (i, [i, d, C.POINTER(C.c_double)]),
+        "amg_debug_wait_timeout_own": (i, [i, i, d, C.POINTER(C.c_double)]),
         "amg_build_hierarchy": (None, [C.POINTER(AmgData), C.POINTER(DcsrMat)]),
         "amg_rebuild_values": (None, [C.POINTER(AmgData), C.POINTER(DcsrMat)]),
         "amg_free": (None, [C.POINTER(AmgData)]),

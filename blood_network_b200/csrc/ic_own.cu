@@ -115,15 +115,20 @@ __device__ __forceinline__ bool own_give_up(const WaitCtl& w, int it, unsigned l
   return *ran_out;
 }
 
+// vector index of the dependency that a code stands for (the wait record's)
+__device__ __forceinline__ int own_dep(int code, const int2* rec, int base) {
+  return code >= 0 ? code : rec[base + ~code].x;
+}
+
 // waits until get() returns a value (bounded; NaN when the wait is abandoned)
-template <class U, class F>
-__device__ __forceinline__ U own_wait(U u, int dep, F get, const WaitCtl& wc, int row) {
+template <class U, class F, class D>
+__device__ __forceinline__ U own_wait(U u, D dep, F get, const WaitCtl& wc, int row) {
   using W = WordOf<typename ValueOf<U>::T>;
   unsigned long long t0 = 0;
   for (int it = 1; u == W::kPending; it++) {
     bool ran_out = false;
     if ((it & (kOwnLook - 1)) == 0 && own_give_up(wc, it, t0, &ran_out)) {
-      if (ran_out) wait_give_up(wc, row, dep, global_ns() - t0);
+      if (ran_out) wait_give_up(wc, row, dep(), global_ns() - t0);
       return W::kNaN;
     }
     u = get();
@@ -200,7 +205,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_own(OwnArgs<T> a) {
               if (w[q] == W::kPending) { dep = c[q]; w[q] = W::kNaN; }
               if (u[q] == W::kPending) { dep = c[q]; u[q] = W::kNaN; }
             }
-            if (ran_out) wait_give_up(a.wc, rec.x, dep, global_ns() - t0);
+            if (ran_out) wait_give_up(a.wc, rec.x, own_dep(dep, a.rec, base), global_ns() - t0);
             pend = false;
           }
         }
@@ -212,7 +217,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_own(OwnArgs<T> a) {
             const int cx = a.xcode[e];
             const unsigned ax = sv0 + (unsigned)(~cx) * (unsigned)sizeof(U);
             auto get = [&] { return cx >= 0 ? ld_relaxed(o + cx) : lds_word<U>(ax); };
-            const U ux = own_wait(get(), cx, get, a.wc, rec.x);
+            const U ux = own_wait(get(), [&] { return own_dep(cx, a.rec, base); }, get, a.wc, rec.x);
             s = sub(s, a.xval[e], ux);
           }
         }
@@ -547,9 +552,81 @@ void run_tri_own(const IChol& ic, bool forward, const T* in, T* out, T* clear, W
   g_launch_count++;
   BN_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
 }
+// The give-up path: a factor whose first row is left out of the forward
+// schedule.  entries 1: a chain; 5: five rows without dependencies, then rows of
+// five, the last of them (past the four that a row keeps at hand) the missing
+// row or the row before.  The vector numbering is the reverse of the rows'.
+static void own_wait_selftest(int n, int entries, double limit_ms, double* elapsed_ms,
+                              cudaStream_t s) {
+  BN_REQUIRE(entries == 1 || entries == 5, BN_ERR_ARG, "wait self-test: 1 or 5 entries");
+  BN_REQUIRE(n > entries && n <= (entries == 1 ? kOwnRows64 : 256), BN_ERR_ARG,
+             "wait self-test: number of rows out of range");
+  BN_REQUIRE(limit_ms > 0.0 && limit_ms <= 10000.0, BN_ERR_ARG,
+             "wait self-test: limit_ms must be in (0, 10000]");
+  std::vector<int> ia(1, 0), ja, inv(n);
+  for (int i = 0; i < n; i++) {
+    if (i >= entries) {
+      for (int q = 1; q < entries; q++) ja.push_back(q);
+      ja.push_back(i == entries ? 0 : i - 1);
+    }
+    ja.push_back(i);
+    ia.push_back((int)ja.size());
+    inv[i] = n - 1 - i;
+  }
+  CSR L;
+  L.alloc(n, n, (int)ja.size(), s, true);
+  L.ia.upload(ia.data(), ia.size());
+  L.ja.upload(ja.data(), ja.size());
+  const std::vector<double> val(ja.size(), 0.5), in(n, 1.0);
+  L.val.upload(val.data(), val.size());
+  DBuf<int> dinv(n, s);
+  DBuf<double> din(n, s), out(n, s);
+  dinv.upload(inv.data(), n);
+  din.upload(in.data(), n);
+  out.fill_bytes(0xff);
+  IChol ic;
+  ic.mode = IChol::kSweepFlags;
+  ic.load(std::move(L), s);
+  ic.remap(dinv.p, s);
+  BN_REQUIRE(ic.own_ready<double>(), BN_ERR_ARG, "wait self-test: the owner form is off");
+  const int first = 1;  // the first step begins behind its first row
+  ic.of.step.upload(&first, 1);
+  ic.wait.limit_ns = (unsigned long long)(limit_ms * 1e6);
+  cudaEvent_t e0, e1;
+  BN_CUDA(cudaEventCreate(&e0));
+  BN_CUDA(cudaEventCreate(&e1));
+  BN_CUDA(cudaEventRecord(e0, s));
+  run_tri_own<double>(ic, true, din.p, out.p, nullptr, ic.wait.ctl(WT_SELFTEST), s);
+  BN_CUDA(cudaEventRecord(e1, s));
+  BN_CUDA(cudaEventSynchronize(e1));
+  float ms = 0.f;
+  cudaEventElapsedTime(&ms, e0, e1);
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  if (elapsed_ms) *elapsed_ms = ms;
+  std::string msg;
+  if (ic.wait.take(s, &msg)) throw Error(BN_ERR_SPIN, "wait self-test: " + msg);
+}
+
 template void run_tri_own<double>(const IChol&, bool, const double*, double*, double*, WaitCtl,
                                   cudaStream_t);
 template void run_tri_own<float>(const IChol&, bool, const float*, float*, float*, WaitCtl,
                                  cudaStream_t);
 
 }  // namespace bn
+
+// See include/amg_b200.h for the contract.
+BN_API int amg_debug_wait_timeout_own(int n, int entries, double limit_ms, double* elapsed_ms) {
+  using namespace bn;
+  try {
+    own_wait_selftest(n, entries, limit_ms, elapsed_ms, cudaStreamPerThread);
+    set_last_error(BN_OK, "");
+    return BN_OK;
+  } catch (const Error& e) {
+    set_last_error(e.code, e.what());
+    return e.code;
+  } catch (const std::exception& e) {
+    set_last_error(BN_ERR_CUDA, e.what());
+    return BN_ERR_CUDA;
+  }
+}

@@ -408,6 +408,12 @@ int amg_network_adjoint_device(void* solver, const amg_network_system* sys, int 
  * launch's device time, about limit_ms.  The device stays usable.  Any
  * other return means the give-up path is broken. */
 int amg_debug_wait_timeout(int n, double limit_ms, double* elapsed_ms);
+/* The same for the form of the sweep whose rows are kept by their blocks (the
+ * chain reversed in the vectors: row r waits for row r+1).  entries 1: the
+ * chain, 2 <= n <= 22000; 5: rows 0..4 without dependencies, later ones with
+ * rows 1..4 and the row before (the first of them the missing row 0),
+ * 6 <= n <= 256. */
+int amg_debug_wait_timeout_own(int n, int entries, double limit_ms, double* elapsed_ms);
 
 /* ichol_solve_noalloc: no counterpart in the reference.  Solves L L^T x = b
  * for an IC(0) factor already in device memory (0-based CSR d_ia[n+1],
