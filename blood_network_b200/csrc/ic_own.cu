@@ -376,13 +376,18 @@ bool IChol::own_ready() const {
 template bool IChol::own_ready<double>() const;
 template bool IChol::own_ready<float>() const;
 
+void IChol::own_drop() {
+  own_blocks = own_rows = 0;
+  of = Own();
+  ob = Own();
+  own_of.release();
+}
+
 // Partition, schedules and packed entries, in the vector numbering inv.  Left
 // unbuilt (own_blocks = 0) where the rows do not fit the blocks' shared
 // memory or where many rows have more than four entries.
 void IChol::own_build(const int* inv, cudaStream_t s) {
-  own_blocks = 0;
-  of = Own();
-  ob = Own();
+  own_drop();
   if (mode != kSweepFlags || n == 0 || nlevels == 0) return;
   const char* e = getenv("BN_IC_OWN");  // 0: the chunked form throughout
   if (e && atoi(e) == 0) return;
@@ -448,7 +453,10 @@ void IChol::own_build(const int* inv, cudaStream_t s) {
     BN_CUDA(cudaStreamSynchronize(s));
     steps = steps > h[0] ? steps : h[0];
     rows = rows > h[1] ? rows : h[1];
-    if (nx > n / 4 + 1024) return;
+    if (nx > n / 4 + 1024) {
+      own_drop();
+      return;
+    }
     w.code.alloc(n, s);
     w.rec.alloc(n, s);
     w.xcode.alloc(nx > 0 ? nx : 1, s);
@@ -458,7 +466,10 @@ void IChol::own_build(const int* inv, cudaStream_t s) {
   if (trace_on())
     fprintf(stderr, "[bn] IC(0) owner form: %d blocks, %d rows a block, %d levels, %d steps a block\n",
             (int)nb, rows, nlevels, steps);
-  if (rows > cap + kOwnSlack) return;
+  if (rows > cap + kOwnSlack) {
+    own_drop();
+    return;
+  }
   own_few = nb < sms;
   own_rows = rows;
   own_blocks = (int)nb;

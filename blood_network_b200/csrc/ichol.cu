@@ -880,7 +880,7 @@ void IChol::load(CSR&& Lf, cudaStream_t s) {
 void IChol::finish(const int* aia, const int* aja, const double* aval, bool numeric,
                    cudaStream_t s) {
   const int g = grid_for(n, 256);
-  own_blocks = 0;
+  own_drop();
   Phase ph_lower("ichol lower", s);
   DBuf<int> flags(1, s);
   flags.zero();
