@@ -986,6 +986,9 @@ void IChol::finish(const int* aia, const int* aja, const double* aval, bool nume
   if (mode == kSweepTiles || (bt && atoi(bt))) {
     build_tiles(true, s);
     build_tiles(false, s);
+  } else {  // not those of the factor before
+    tf = Tiles();
+    tb = Tiles();
   }
   if (mode == kSweepSlab || mode == kSweepSlabW) {
     build_slab_partition(s);
