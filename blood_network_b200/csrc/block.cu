@@ -321,10 +321,19 @@ k_gsm(const int* __restrict__ ia, const int* __restrict__ ja, const T* __restric
   const bool c0 = lane < K, c1 = lane + 32 < K;
   block_rows<T, SPLIT, PAIR>(ia, ja, a, r0, nshort, 0, true, X, K, [&](int t, T s0, T s1, T d) {
     const int i = r0 + t;
-    T b0, b1;
-    row_load<T, PAIR>(B + (size_t)i * K, lane, c0, c1, b0, b1);
-    row_store<T, PAIR>(OUT ? OUT + (size_t)t * K : X + (size_t)i * K, lane, c0, c1,
-                       bsub(b0, s0) / d, bsub(b1, s1) / d);
+    const T* br = B + (size_t)i * K;
+    T* o = OUT ? OUT + (size_t)t * K : X + (size_t)i * K;
+    if (PAIR || (sizeof(T) == 4 && K > 32)) {
+      T b0, b1;
+      row_load<T, PAIR>(br, lane, c0, c1, b0, b1);
+      row_store<T, PAIR>(o, lane, c0, c1, bsub(b0, s0) / d, bsub(b1, s1) / d);
+    } else {
+      // Made by every lane the second division costs FP64 4 more registers and a
+      // third of the kernel (5k rows, 33 columns: 6.6 us, 8.7), and is in vain up to
+      // 32 columns; FP32 beyond is 1 % of a solve faster without the branches.
+      if (c0) o[lane] = bsub(br[lane], s0) / d;
+      if (c1) o[lane + 32] = bsub(br[lane + 32], s1) / d;
+    }
   });
 }
 
