@@ -881,6 +881,7 @@ void IChol::finish(const int* aia, const int* aja, const double* aval, bool nume
                    cudaStream_t s) {
   const int g = grid_for(n, 256);
   own_drop();
+  own_unfit = 0;
   Phase ph_lower("ichol lower", s);
   DBuf<int> flags(1, s);
   flags.zero();
@@ -1024,8 +1025,7 @@ void IChol::remap(const int* inv, cudaStream_t s) {
   }
   if (inv) {  // a solver's sweeps; a factor solved once does not repay the schedule
     Phase ph("ichol owner form", s);
-    own_build(inv, s);
-    own_values(s);
+    own_number(inv, s);
   }
 }
 

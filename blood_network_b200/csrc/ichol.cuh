@@ -117,6 +117,8 @@ struct IChol {
   DBuf<int> own_of;               // natural row -> block
   int own_blocks = 0, own_rows = 0, own_limit = 0;  // blocks (0: not built), rows of the fullest
   bool own_few = false;           // fewer blocks than SMs: smaller blocks
+  int own_unfit = 0;              // precisions (1 FP64, 2 FP32) that it does not suit
+  void own_number(const int* inv, cudaStream_t s);
   void own_drop();
   void own_build(const int* inv, cudaStream_t s);
   void own_values(cudaStream_t s);

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from blood_network_b200 import amg
-from test_gpu_solve_paths import _random_spd, _vascular
+from test_gpu_solve_paths import OWN_CASES, _random_spd, _vascular
 
 pytestmark = pytest.mark.gpu
 
@@ -108,3 +108,22 @@ def test_owner_sweeps_in_the_precision_at_hand():
         s.bench_kernel(3, precision=1, reps=1)
         check(s, first)
         s.close()
+
+
+@pytest.mark.parametrize("precision", [amg.PREC_FP64, amg.PREC_MIXED])
+@pytest.mark.parametrize("name", sorted(OWN_CASES))
+def test_owner_schedule_over_smoothers(name, precision, monkeypatch):
+    """A new smoother numbers the vectors anew; the sweeps' schedule stays and gives
+    the chunked sweeps' bits after each change."""
+    n, ia, ja, val = OWN_CASES[name]()
+    g = np.random.default_rng(n).standard_normal(n)
+    out = {}
+    for own in "10":
+        monkeypatch.setenv("BN_IC_OWN", own)
+        s = amg.AMGSolver(n, ia, ja, val, precision=precision, min_size=30)
+        out[own] = []
+        for smoother in (amg.SMOOTHER_GS, amg.SMOOTHER_JACOBI, amg.SMOOTHER_CF_GS):
+            s.set_smoother(smoother)
+            out[own].append(s.precond(g).tobytes())
+        s.close()
+    assert out["1"] == out["0"] and len(set(out["1"])) == 3
