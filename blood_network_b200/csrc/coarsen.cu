@@ -426,11 +426,10 @@ static int count_c(const int* cf, int n, cudaStream_t s) {
 // own drawing and uploading from the host took 15 ms of a 1M-row PMIS level,
 // 27 ms over the hierarchy; here 5.3).  Device draws pay from some ten
 // thousand points on: the jump matrices cost the host half a millisecond.
-constexpr int kHostDraws = 32768;
 const int* RandDraws::first(int n, bool host_ok, cudaStream_t s) {
   if ((size_t)n <= d.n) return d.p;
   d.alloc(n, s);
-  if (host_ok && n <= kHostDraws) {
+  if (host_ok && n <= host_max) {
     std::vector<int> h(n);
     srand(12345);
     for (int i = 0; i < n; i++) h[i] = rand();

@@ -19,10 +19,11 @@ void strength(const CSR& A, double theta, CSR& S, int* max_lam, cudaStream_t s);
 enum Coarsening : int { COARSEN_RS = 0, COARSEN_PMIS = 1, COARSEN_HMIS = 2 };
 // cf[i] = +1 (C) / -1 (F); returns the number of C points.
 // rand() draws after srand(12345) on the device, kept for the levels of one
-// hierarchy.  host_ok: short sequences may come from the C library itself
-// (which moves its state).
+// hierarchy.  host_ok: sequences of up to host_max may come from the C library
+// itself (which moves its state).
 struct RandDraws {
   DBuf<int> d;
+  int host_max = 32768;
   const int* first(int n, bool host_ok, cudaStream_t s);
 };
 int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s, RandDraws& draws);
