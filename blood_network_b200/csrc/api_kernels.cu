@@ -111,17 +111,12 @@ BN_API void rs_standard_interpolation_sparsity(const dcsr_mat* S, const int* cf,
   });
 }
 
-// A solver's matrices hold a column once per row (it refuses others); a
-// caller's need not.  Columns are points, so both matrices are n x n.
-static bool distinct_rows(const dcsr_mat* A, CSR& dA, const dcsr_mat* S, CSR& dS,
-                          cudaStream_t s) {
-  BN_REQUIRE(A->ia[A->row] <= A->nnz && S->ia[S->row] <= S->nnz, BN_ERR_ARG,
-             "row pointers beyond the entries");
-  dA.m = dA.n;
-  dS.m = dS.n;
-  dA.nnz = A->ia[A->row];  // entries of the rows; the arrays may be longer
-  dS.nnz = S->ia[S->row];
-  return distinct_columns(dA, dS, s);
+// Columns are points, so both matrices are n x n; the arrays may be longer than
+// the rows' entries.
+static void as_point_matrix(const dcsr_mat* h, CSR& d) {
+  BN_REQUIRE(h->ia[h->row] <= h->nnz, BN_ERR_ARG, "row pointers beyond the entries");
+  d.m = d.n;
+  d.nnz = h->ia[h->row];
 }
 
 BN_API void rs_standard_interpolation_values(const dcsr_mat* A, const dcsr_mat* S, const int* cf,
@@ -135,7 +130,9 @@ BN_API void rs_standard_interpolation_values(const dcsr_mat* A, const dcsr_mat* 
     to_device(P, dP, s);
     DBuf<int> dcf(n > 0 ? n : 1, s);
     dcf.upload(cf, n);
-    interpolation_values(dA, dS, dcf.p, dP, s, distinct_rows(A, dA, S, dS, s));
+    as_point_matrix(A, dA);
+    as_point_matrix(S, dS);
+    interpolation_values(dA, dS, dcf.p, dP, s, false);  // rows as the caller has them
     dP.val.download(P->val, P->nnz);
     BN_CUDA(cudaStreamSynchronize(s));
   });
@@ -153,7 +150,9 @@ BN_API void rs_standard_interpolation(const dcsr_mat* A, const dcsr_mat* S, cons
     dcf.upload(cf, n);
     int nc = 0;
     for (int i = 0; i < n; i++) nc += (cf[i] == 1);
-    interpolation(dA, dS, dcf.p, nc, dP, s, distinct_rows(A, dA, S, dS, s));
+    as_point_matrix(A, dA);
+    as_point_matrix(S, dS);
+    interpolation(dA, dS, dcf.p, nc, dP, s, false);
     to_host(dP, P, s);
   });
 }

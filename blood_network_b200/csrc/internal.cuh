@@ -32,14 +32,13 @@ int coarsen(const CSR& S, int method, int max_lam, int* cf, cudaStream_t s, Rand
 void pmis_rand_state(int n);
 
 // ---- interp.cu
-// distinct: no row of A or S holds a column twice (true of a solver's matrices).
+// distinct: no row of A or S holds a column twice (true of a solver's matrices);
+// otherwise that is looked for.
 void interpolation(const CSR& A, const CSR& S, const int* cf, int n_coarse, CSR& P,
                    cudaStream_t s, bool distinct = true);
 void interpolation_pattern(const CSR& S, const int* cf, int n_coarse, CSR& P, cudaStream_t s);
 void interpolation_values(const CSR& A, const CSR& S, const int* cf, CSR& P, cudaStream_t s,
                           bool distinct = true);
-// whether no row of A or S holds a column twice
-bool distinct_columns(const CSR& A, const CSR& S, cudaStream_t s);
 
 // ---- rap.cu
 void rap(const CSR& R, const CSR& A, const CSR& P, CSR& Ac, cudaStream_t s);

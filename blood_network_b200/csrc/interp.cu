@@ -587,23 +587,33 @@ __global__ void k_interp_values(const int* __restrict__ aia, const int* __restri
 }
 
 // flag[0] = 1: a row of at most kTwiceRow entries holds a column twice;
-// flag[1] = 1: there are longer rows.  A warp per row, all pairs (1M-row network,
-// both matrices: 0.4 ms of the call's 10; all rows by the transpose 3).
-constexpr int kTwiceRow = 512;
+// flag[1] = 1: there are longer rows.  All pairs: a thread per row of up to 16
+// entries, the warp together for a longer one.
+constexpr int kTwiceRow = 512, kTwiceThread = 16;
 __global__ void k_twice(const int* __restrict__ ia, const int* __restrict__ ja, int n,
                         int* __restrict__ flag) {
-  const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-    const int k0 = ia[i], k1 = ia[i + 1];
-    if (k1 - k0 > kTwiceRow) {
-      if (lane == 0) flag[1] = 1;
-      continue;
-    }
+  const int lane = threadIdx.x & 31, threads = gridDim.x * blockDim.x;
+  for (int r0 = blockIdx.x * blockDim.x + threadIdx.x - lane; r0 < n; r0 += threads) {
+    const int i = r0 + lane;
+    const int k0 = i < n ? ia[i] : 0, k1 = i < n ? ia[i + 1] : 0;
     bool twice = false;
-    for (int base = k0; base < k1; base += 32) {
-      const int j = base + lane < k1 ? ja[base + lane] : -1 - lane;  // columns are not negative
-      twice |= __popc(__match_any_sync(0xffffffffu, j)) > 1;
-      for (int k = k0; k < base; k++) twice |= ja[k] == j;
+    if (k1 - k0 <= kTwiceThread) {
+      for (int k = k0 + 1; k < k1; k++) {
+        const int j = ja[k];
+        for (int q = k0; q < k; q++) twice |= ja[q] == j;
+      }
+    } else if (k1 - k0 > kTwiceRow) {
+      flag[1] = 1;
+    }
+    unsigned mid = __ballot_sync(0xffffffffu, k1 - k0 > kTwiceThread && k1 - k0 <= kTwiceRow);
+    for (; mid; mid &= mid - 1) {
+      const int q0 = __shfl_sync(0xffffffffu, k0, __ffs(mid) - 1);
+      const int q1 = __shfl_sync(0xffffffffu, k1, __ffs(mid) - 1);
+      for (int base = q0; base < q1; base += 32) {
+        const int j = base + lane < q1 ? ja[base + lane] : -1 - lane;  // columns are not negative
+        twice |= __popc(__match_any_sync(0xffffffffu, j)) > 1;
+        for (int k = q0; k < base; k++) twice |= ja[k] == j;
+      }
     }
     if (twice) flag[0] = 1;
   }
@@ -618,34 +628,36 @@ __global__ void k_twice_t(const int* __restrict__ tia, const int* __restrict__ t
       if (tja[k] == tja[k - 1]) flag[0] = 1;
 }
 
-bool distinct_columns(const CSR& A, const CSR& S, cudaStream_t s) {
-  const CSR* ms[2] = {&A, &S};
-  DBuf<int> flags(4, s);
-  flags.zero();
-  for (int q = 0; q < 2; q++)
-    if (ms[q]->n > 0)
-      BN_LAUNCH(k_twice, grid_for((long long)ms[q]->n * 32, 256, 16), 256, 0, s, ms[q]->ia.p,
-                ms[q]->ja.p, ms[q]->n, flags.p + 2 * q);
-  int h[4];
-  flags.download(h, 4);
-  BN_CUDA(cudaStreamSynchronize(s));
-  if (h[0] || h[2]) return false;
-  for (int q = 0; q < 2; q++) {
-    if (!h[2 * q + 1]) continue;
-    CSR T;
-    transpose(*ms[q], T, s, false);
-    BN_LAUNCH(k_twice_t, grid_for((long long)T.n * 32, 256, 16), 256, 0, s, T.ia.p, T.ja.p, T.n,
-              flags.p);
-    if (read_scalar(flags.p, s)) return false;
-  }
-  return true;
+// flags 0 and 1 of A, 2 and 3 of S as k_twice leaves them
+static void look_for_twice(const CSR& M, int* flags, cudaStream_t s) {
+  if (M.n > 0)
+    BN_LAUNCH(k_twice, grid_for(M.n, 128), 128, 0, s, M.ia.p, M.ja.p, M.n, flags);
+}
+static bool long_rows_hold_twice(const CSR& M, cudaStream_t s) {
+  CSR T;
+  transpose(M, T, s, false);
+  DBuf<int> flag(1, s);
+  flag.zero();
+  BN_LAUNCH(k_twice_t, grid_for((long long)T.n * 32, 256, 16), 256, 0, s, T.ia.p, T.ja.p, T.n, flag.p);
+  return read_scalar(flag.p, s) != 0;
 }
 
 void interpolation_values(const CSR& A, const CSR& S, const int* cf, CSR& P, cudaStream_t s,
                           bool distinct) {
   if (A.n == 0) return;
   const int n = A.n;
+  DBuf<int> hubidx(n, s), hubrows(n, s), ctr(6, s);
+  ctr.zero();
   if (!distinct) {
+    look_for_twice(A, ctr.p + 2, s);
+    look_for_twice(S, ctr.p + 4, s);
+  }
+  BN_LAUNCH(k_hub_mark, grid_for(n, 256), 256, 0, s, A.ia.p, n, hubidx.p, hubrows.p, ctr.p);
+  int hn[6];
+  ctr.download(hn, 6);
+  BN_CUDA(cudaStreamSynchronize(s));
+  if (hn[2] || hn[4] || (hn[3] && long_rows_hold_twice(A, s)) ||
+      (hn[5] && long_rows_hold_twice(S, s))) {
     // The warp and block kernels and the hub tables count on one entry per
     // column (they add a neighbour's entries in parallel and keep at most one
     // per strong point); a thread per row takes the entries as they come.
@@ -655,10 +667,7 @@ void interpolation_values(const CSR& A, const CSR& S, const int* cf, CSR& P, cud
               S.ja.p, cf, n, wide.p, P.ia.p, P.val.p, nullptr, nullptr, nullptr, nullptr);
     return;
   }
-  DBuf<int> hubidx(n, s), hubrows(n, s), ctr(2, s);
-  ctr.zero();
-  BN_LAUNCH(k_hub_mark, grid_for(n, 256), 256, 0, s, A.ia.p, n, hubidx.p, hubrows.p, ctr.p);
-  const int nh = read_scalar(ctr.p, s);
+  const int nh = hn[0];
   DBuf<int> hoff((size_t)nh + 1, s), keys, vals;
   if (nh > 0) {
     hoff.zero();
@@ -676,7 +685,6 @@ void interpolation_values(const CSR& A, const CSR& S, const int* cf, CSR& P, cud
   BN_LAUNCH(k_interp_values, grid_for(n, 128), 128, 0, s, A.ia.p, A.ja.p, A.val.p, S.ia.p,
             S.ja.p, cf, n, wide.p, P.ia.p, P.val.p, nh > 0 ? hubidx.p : nullptr, hoff.p, keys.p,
             vals.p);
-  int hn[2];
   ctr.download(hn, 2);
   BN_CUDA(cudaStreamSynchronize(s));
   const int nw = hn[0];
