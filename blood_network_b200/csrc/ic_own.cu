@@ -51,8 +51,10 @@ namespace {
 
 // Threads of a block: with fewer blocks than SMs 8 warps (few warps leave the
 // one on the chain the issue slots: 300k rows FP64 299 us, 16 warps 324), else
-// 16, in FP32 32 (4M rows: 850 us with 16, 692 with 32; FP64 does not fit the
-// registers of 32).
+// 16, in FP32 32 (4M rows: 850 us with 16, 692 with 32).  FP64 takes 70 registers
+// a thread, so 28 warps are the most that fit; its two sweeps in microseconds at
+// 2M / 3M / 4M rows: 16 warps 642 / 834 / 1073, 24 warps 681 / 889 / 1205, 28
+// warps 608 / 781 / 1271 (the chunked form 799 / 1022 / 1074).
 constexpr int kOwnFew = 256, kOwnMany64 = 512, kOwnMany32 = 1024;
 constexpr int kOwnLanes = 4;         // rows of one level per warp that the block count aims at
 constexpr int kOwnSlack = 640;       // rows per block kept free for uneven shares
@@ -60,7 +62,9 @@ constexpr int kDealt = 512;          // rows of one level in a block's range: ab
 // Rows per block up to which the form is used, chunked form -> this one:
 // FP64 820 -> 641 us at 13,600 (2M rows), 1046 -> 835 at 20,300 (3M),
 // 1095 -> 1077 at 27,000 (4M); FP32 978 -> 692 at 27,000, 1240 -> 812 at
-// 40,700 (6M), 1356 -> 1520 at 54,200 (8M).
+// 40,700 (6M), 1356 -> 1520 at 54,200 (8M).  The blocks are counted by the levels
+// and the shared memory (own_build), so a deep, narrow factor can pass the line
+// with SMs left over; it keeps the chunked form.
 constexpr int kOwnRows64 = 22000, kOwnRows32 = 45000;
 constexpr int kNoEntry = (int)0x80000000;
 

@@ -192,7 +192,7 @@ constexpr int kBlkThreads = 256, kBlkTable = 2 * kBlockMaxS;
 struct InterpBlock {
   int key[kBlkTable];      // column, -1 empty
   int slot[kBlkTable];     // C: rank among the C points of S_i; F: -1
-  int fk[kBlockMaxS];      // entries of A_i that are strong F points, in order
+  int fk[kBlockMaxS];      // entries of A_i that are strong F points, in order (a column once)
   double den[kBlockMaxS];  // their denominators
   double num[kBlockMaxS];  // the row of P by slot
   double weak[kBlkThreads];
@@ -206,7 +206,7 @@ __device__ __forceinline__ int blk_find(const InterpBlock& t, int m, bool* in) {
     at = (at + 1) & (kBlkTable - 1);
   }
 }
-// inclusive rank of the threads with flag set, in thread order, plus the block's total
+// how many threads before this one have flag set, and the block's total
 __device__ __forceinline__ int blk_rank(bool flag, int* wsum, int* total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned b = __ballot_sync(0xffffffffu, flag);

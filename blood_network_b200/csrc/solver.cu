@@ -65,7 +65,8 @@ constexpr long long kSmallLevelNnz = 65536;
 // here, less than the 4-5 us of a launch over all of them; beyond, the entries
 // count.  Whole solves, microseconds, without the tail / line at 65k / 140k /
 // 262k entries: 20k FP64 4438 / 3924 / 3851 / 3850, one preconditioner at 75k
-// 1033 / 971 / 945 / 1000, 64 packed networks 18134 / 16631 / 16980 / 16987.
+// 1033 / 971 / 945 / 1000, 64 packed networks 18134 / 16631 / 16980 / 16987: the
+// line lies between the two that are best, itself not timed against them.
 constexpr long long kTailNnz = 100000;
 constexpr int kTailRows = 32768;
 
@@ -495,7 +496,8 @@ static std::vector<int> host_ia(const CSR& M, cudaStream_t s) {
 // entries; 4M 1, 2, 4, 16 for 5, 9, 17, 39 entries; 20M mixed 1, 1, 4, 16 for
 // 5, 10, 20, 48.  One lane up to 12 entries, 8 up to 48 and 32 beyond for every
 // size (as it was) -> those choices: one solve at 75k 7.03 -> 6.52 ms, 4M 32.0 ->
-// 31.3, 20M 94.2 -> 91.9.
+// 31.3, 20M 94.2 -> 91.9.  (Four lanes on short rows up to twice the line rest on
+// the 75k network's finest level alone.)
 constexpr int kGsFewRows = 65536;
 static int gs_lanes(int n, double avg) {
   if (n <= kGsFewRows) {
@@ -1346,7 +1348,9 @@ void l1_row_norms(const CSR& A, double* d_out, cudaStream_t s) {
 // blocks take slots from the running kernel.  Without -> with, milliseconds:
 // one preconditioner at 75k 0.949 -> 0.807, 300k mixed 10.01 -> 9.43, 1.43M rows
 // mixed 16.66 -> 16.02, 500k FP64 gradient 79.8 -> 78.9; 2M FP64 22.86 -> 23.27,
-// 4M 29.6 -> 30.3, 20M mixed 98.5 -> 103.6.
+// 4M 29.6 -> 30.3, 20M mixed 98.5 -> 103.6.  Around the line, FP64: 1.2M 19.91 ->
+// 19.88, 1.45M 22.30 -> 22.42, 1.8M 23.00 -> 23.14; mixed: 16.98 -> 16.29, 19.37 ->
+// 18.60, 19.83 -> 19.16.
 constexpr int kPdlRows = 1600000;
 
 // z = M r for the PCG: r -> z (captured once per precision as a CUDA graph)
@@ -2316,9 +2320,11 @@ BN_API unsigned long long amg_b200_launch_count(void) { return bn::g_launch_coun
 // Per level, times the candidate kernels of the solve phase on the level's
 // own operators and keeps the fastest:
 //  * SpMV, restriction and prolongation (A, R, P): the row-tile kernel with
-//    256, 128, 64 or 32 rows per tile (groups 0-3) or 4, 8 or 32 lanes per
-//    row (the rows-per-warp / vector-width choice of the row-group kernels);
-//  * Gauss-Seidel colour classes: 1, 8 or 32 lanes per row.
+//    256, 128, 64 or 32 rows per tile (groups 0-3), staged 256-row tiles (5) or
+//    4, 8, 16 or 32 lanes per row (the rows-per-warp / vector-width choice of
+//    the row-group kernels);
+//  * Gauss-Seidel colour classes: staged row tiles (0) or 1, 2, 4, 8, 16 or 32
+//    lanes per row.
 // Each candidate computes every row sum over the row's entries (tile
 // kernel: in storage order; row groups: lane strides then a fixed shuffle
 // tree), so the choice changes rounding only.  Timed in the precision the

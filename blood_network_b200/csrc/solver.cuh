@@ -148,8 +148,8 @@ struct Solver {
   void choose_tail();
   template <class T> void ensure_tail();
   template <class T> void smooth(int l, const T* bb, T* xl, bool forward);
-  // zero_guess: xl holds zeros on entry (every call inside the
-  // preconditioner), which allows the split first sweep
+  // zero_guess: the initial guess is zero, whatever xl holds (every call inside
+  // the preconditioner), which allows the split first sweep; else it is xl
   template <class T> void backslash(int l, const T* bb, T* xl, bool zero_guess);
   void build_split(Level& L);
   template <class T> void fwdslash(int l, const T* bb, T* xl);
