@@ -4,6 +4,8 @@
 #pragma once
 #include "common.cuh"
 
+#include <functional>
+
 #include <vector>
 
 namespace bn {
@@ -75,7 +77,7 @@ constexpr int kSpinHardCap = 1 << 27;    // polls: a last bound should the clock
 //   [0] abort word: set by the first wait that gives up
 //   [1] tag of that kernel (WaitTag)
 //   [2] the waiting row (vector index)
-//   [3] the dependency it waited for (vector index)
+//   [3] the dependency it waited for (vector index; ic_own.cu: ~slot of the row's block)
 //   [4] how long it waited, microseconds
 constexpr int kWaitWords = 8;
 enum WaitTag : int { WT_IC_FWD = 1, WT_IC_BWD = 2, WT_GS_ORDERED = 3, WT_SELFTEST = 4 };
@@ -190,8 +192,10 @@ struct WaitRecord {
   }
   WaitCtl ctl(int tag) const { return WaitCtl{rec.p, limit_ns, tag}; }
   // 0, or BN_ERR_SPIN with *msg describing the wait that gave up; the
-  // record is cleared (synchronous on s).
-  int take(cudaStream_t s, std::string* msg);
+  // record is cleared (synchronous on s).  dep_row(tag, row, dep): the vector
+  // index of a dependency that the record holds in another form.
+  int take(cudaStream_t s, std::string* msg,
+           const std::function<int(int, int, int)>& dep_row = nullptr);
   static unsigned long long default_limit_ns();
 };
 

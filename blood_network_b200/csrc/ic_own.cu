@@ -51,10 +51,10 @@ namespace {
 
 // Threads of a block: with fewer blocks than SMs 8 warps (few warps leave the
 // one on the chain the issue slots: 300k rows FP64 299 us, 16 warps 324), else
-// 16, in FP32 32 (4M rows: 850 us with 16, 692 with 32).  FP64 takes 70 registers
+// 16, in FP32 32 (4M rows: 850 us with 16, 692 with 32).  FP64 takes 68 registers
 // a thread, so 28 warps are the most that fit; its two sweeps in microseconds at
-// 2M / 3M / 4M rows: 16 warps 642 / 834 / 1073, 24 warps 681 / 889 / 1205, 28
-// warps 608 / 781 / 1271 (the chunked form 799 / 1022 / 1074).
+// 2M / 3M / 4M rows: 16 warps 637 / 830 / 1081, 24 warps 679 / 885 / 1212, 28
+// warps 604 / 775 / 1258 (the chunked form 797 / 1018 / 1069).
 constexpr int kOwnFew = 256, kOwnMany64 = 512, kOwnMany32 = 1024;
 constexpr int kOwnLanes = 4;         // rows of one level per warp that the block count aims at
 constexpr int kOwnSlack = 640;       // rows per block kept free for uneven shares
@@ -119,20 +119,18 @@ __device__ __forceinline__ bool own_give_up(const WaitCtl& w, int it, unsigned l
   return *ran_out;
 }
 
-// vector index of the dependency that a code stands for (the wait record's)
-__device__ __forceinline__ int own_dep(int code, const int2* rec, int base) {
-  return code >= 0 ? code : rec[base + ~code].x;
-}
-
-// waits until get() returns a value (bounded; NaN when the wait is abandoned)
-template <class U, class F, class D>
-__device__ __forceinline__ U own_wait(U u, D dep, F get, const WaitCtl& wc, int row) {
+// Waits until get() returns a value (bounded; NaN when the wait is abandoned).
+// The record takes the dependency's code as it is: naming its row here, cold as
+// the path is, made the sweep 9 % slower (1.43M rows FP32: 76 us, 83), so the
+// host does (own_dep_row).
+template <class U, class F>
+__device__ __forceinline__ U own_wait(U u, int dep, F get, const WaitCtl& wc, int row) {
   using W = WordOf<typename ValueOf<U>::T>;
   unsigned long long t0 = 0;
   for (int it = 1; u == W::kPending; it++) {
     bool ran_out = false;
     if ((it & (kOwnLook - 1)) == 0 && own_give_up(wc, it, t0, &ran_out)) {
-      if (ran_out) wait_give_up(wc, row, dep(), global_ns() - t0);
+      if (ran_out) wait_give_up(wc, row, dep, global_ns() - t0);
       return W::kNaN;
     }
     u = get();
@@ -209,7 +207,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_own(OwnArgs<T> a) {
               if (w[q] == W::kPending) { dep = c[q]; w[q] = W::kNaN; }
               if (u[q] == W::kPending) { dep = c[q]; u[q] = W::kNaN; }
             }
-            if (ran_out) wait_give_up(a.wc, rec.x, own_dep(dep, a.rec, base), global_ns() - t0);
+            if (ran_out) wait_give_up(a.wc, rec.x, dep, global_ns() - t0);
             pend = false;
           }
         }
@@ -221,7 +219,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tri_own(OwnArgs<T> a) {
             const int cx = a.xcode[e];
             const unsigned ax = sv0 + (unsigned)(~cx) * (unsigned)sizeof(U);
             auto get = [&] { return cx >= 0 ? ld_relaxed(o + cx) : lds_word<U>(ax); };
-            const U ux = own_wait(get(), [&] { return own_dep(cx, a.rec, base); }, get, a.wc, rec.x);
+            const U ux = own_wait(get(), cx, get, a.wc, rec.x);
             s = sub(s, a.xval[e], ux);
           }
         }
@@ -605,6 +603,24 @@ void run_tri_own(const IChol& ic, bool forward, const T* in, T* out, T* clear, W
   g_launch_count++;
   BN_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
 }
+// Vector index of the dependency that a wait record of a sweep holds: itself, or
+// for a value of the waiting row's own block the row at that slot of the block.
+int IChol::own_dep_row(bool forward, int row, int dep, cudaStream_t s) const {
+  const Own& w = forward ? of : ob;
+  if (dep >= 0 || own_blocks == 0) return dep;
+  std::vector<int2> rec(n);
+  std::vector<int> base((size_t)own_blocks + 1);
+  w.rec.download(rec.data(), n);
+  w.base.download(base.data(), base.size());
+  BN_CUDA(cudaStreamSynchronize(s));
+  for (int b = 0; b < own_blocks; b++)
+    for (int p = base[b]; p < base[b + 1]; p++) {
+      const int at = base[b] + ~dep;
+      if (rec[p].x == row) return at < base[b + 1] ? rec[at].x : dep;
+    }
+  return dep;
+}
+
 // The give-up path: a factor whose first row is left out of the forward
 // schedule.  entries 1: a chain; 5: five rows without dependencies, then rows of
 // five, the last of them (past the four that a row keeps at hand) the missing
@@ -658,7 +674,8 @@ static void own_wait_selftest(int n, int entries, double limit_ms, double* elaps
   cudaEventDestroy(e1);
   if (elapsed_ms) *elapsed_ms = ms;
   std::string msg;
-  if (ic.wait.take(s, &msg)) throw Error(BN_ERR_SPIN, "wait self-test: " + msg);
+  if (ic.wait.take(s, &msg, [&](int, int row, int dep) { return ic.own_dep_row(true, row, dep, s); }))
+    throw Error(BN_ERR_SPIN, "wait self-test: " + msg);
 }
 
 template void run_tri_own<double>(const IChol&, bool, const double*, double*, double*, WaitCtl,

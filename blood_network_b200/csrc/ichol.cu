@@ -1283,7 +1283,10 @@ template void IChol::solve<float>(const float*, float*, float*, cudaStream_t);
 void IChol::check_waits(cudaStream_t s) {
   if (!wait.rec.p) return;
   std::string msg;
-  if (wait.take(s, &msg)) throw Error(BN_ERR_SPIN, "IC(0) solve: " + msg);
+  if (wait.take(s, &msg, [&](int tag, int row, int dep) {
+        return own_dep_row(tag == WT_IC_FWD, row, dep, s);
+      }))
+    throw Error(BN_ERR_SPIN, "IC(0) solve: " + msg);
 }
 
 unsigned long long WaitRecord::default_limit_ns() {
@@ -1298,7 +1301,8 @@ unsigned long long WaitRecord::default_limit_ns() {
   return v;
 }
 
-int WaitRecord::take(cudaStream_t s, std::string* msg) {
+int WaitRecord::take(cudaStream_t s, std::string* msg,
+                     const std::function<int(int, int, int)>& dep_row) {
   int h[kWaitWords];
   rec.download(h, kWaitWords);
   BN_CUDA(cudaStreamSynchronize(s));
@@ -1307,6 +1311,7 @@ int WaitRecord::take(cudaStream_t s, std::string* msg) {
   static const char* names[] = {"?", "forward IC(0) sweep", "backward IC(0) sweep",
                                 "ordered Gauss-Seidel sweep", "wait self-test"};
   const int tag = (h[1] >= 1 && h[1] <= 4) ? h[1] : 0;
+  if (dep_row) h[3] = dep_row(tag, h[2], h[3]);
   char buf[256];
   snprintf(buf, sizeof buf,
            "a bounded dependency wait ran out (%s: row %d waited %.3f ms for row %d; the "

@@ -123,6 +123,7 @@ struct IChol {
   void own_build(const int* inv, cudaStream_t s);
   void own_values(cudaStream_t s);
   void own_want(cudaStream_t s);
+  int own_dep_row(bool forward, int row, int dep, cudaStream_t s) const;
   template <class T> bool own_ready() const;
   DBuf<int> fia, fja, fsrc; // forward rows (level order)
   DBuf<int> bia, bja, bsrc; // backward rows (reverse level order)
